@@ -227,21 +227,25 @@ class _Handle:
 
 
 class _ListBuffers:
-    """Device buffers of a program that keeps its neighbour list in a fixed capacity, a little above the expected pairs."""
+    """Device buffers of a program that keeps its neighbour list in a fixed capacity, a little above the expected pairs,
+    sorted by the lower particle of a pair and then the other (both of one system, so that it is less than `span` away)."""
 
     def __init__(self, case, n):
         self.cap = int(1.05 * _pairs(case)) + 8192
-        self.end = n * n
-        self.i, self.j, self.key = (torch.empty(self.cap, dtype=torch.int64, device="cuda") for _ in range(3))
+        self.span = case["nmax"] if case["how"] == "batch" else n
+        self.end = n * self.span
+        narrow = self.end < 2 ** 31
+        self.i, self.j = (torch.empty(self.cap, dtype=torch.int64, device="cuda") for _ in range(2))
+        self.key = torch.empty(self.cap, dtype=torch.int32 if narrow else torch.int64, device="cuda")
         self.d = torch.empty(self.cap, dtype=_dt(case), device="cuda")
 
-    def fill(self, L, h, count, n):
-        """The list in the order of its pairs, min(i, j) n + max(i, j), the rest of the buffers after it as n n and 0."""
+    def fill(self, L, h, count):
+        """The list in the order of its pairs as lower * span + (upper - lower), and 0 for the rest of the distances."""
         status = L.clm_nl_fetch(h, self.i.data_ptr(), self.j.data_ptr(), self.d.data_ptr(), self.cap, 0, 1)
         if status:
             raise RuntimeError("clm status %d" % status)
         i, j = self.i[:count], self.j[:count]
-        torch.add(torch.maximum(i, j), torch.minimum(i, j), alpha=n, out=self.key[:count])
+        self.key[:count] = torch.add((i - j).abs_(), torch.minimum(i, j), alpha=self.span)
         self.key[count:] = self.end
         self.d[count:] = 0
         key, at = torch.sort(self.key)
@@ -278,7 +282,7 @@ def run(state):
         sys.update(positions=inp["x"])
         lists, energy = sys.run(*state["ops"])
         h = sys._handle
-        return {"counts": lists.counts, "energy": energy, "list": state["list"].fill(h.L, h.h, lists.total, int(inp["off"][-1]))}
+        return {"counts": lists.counts, "energy": energy, "list": state["list"].fill(h.L, h.h, lists.total)}
     if case["how"] == "python":
         sys = state["sys"]
         sys.update(xpositions=inp["x"], ypositions=inp.get("y"))
@@ -287,7 +291,7 @@ def run(state):
     h = state["handle"]
     h.step()
     if case["how"] == "nl":
-        return state["list"].fill(h.L, h.h, h.o.count, case["n"])
+        return state["list"].fill(h.L, h.h, h.o.count)
     if case["op"] == "rhist":
         return {"counts": h.hc, "sums": h.hs}
     out = {"energy": h.o.scalar}
