@@ -1138,20 +1138,31 @@ template <class T> int build_set(Handle& h, int set, const Geometry<T>& g) {
 
 // Reads the device totals of the last build of every set (after the caller synchronized the stream
 // through `staged`, which the caller filled with enqueue_build_totals) and checks the error word.
-int enqueue_build_totals(Handle& h) {
+Totals build_totals(Handle& h) {
+  Totals t;
+  t.n = 0;
+  auto add = [&](const int* src, int at) {
+    t.src[t.n] = src;
+    t.dst[t.n++] = h.pinned + at;
+  };
   for (int s = 0; s < h.nsets; s++) {
     SetData& S = h.sets[s];
     if (!S.pending) continue;
     // the number of copies: the copy-offset scan's total, or (counting build) the last cell start
-    const int* copies = S.counted ? S.cell_start.as<int>() + S.ncells : S.copy_off.as<int>() + S.n;
-    CLM_CUDA_TRY(h, cudaMemcpyAsync(h.pinned + 32 + 2 * s, copies, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
-    CLM_CUDA_TRY(h, cudaMemcpyAsync(h.pinned + 33 + 2 * s, S.real_scan.as<int>() + S.ncells, sizeof(int),
-                                    cudaMemcpyDeviceToHost, h.stream));
-    if (S.counted)
-      CLM_CUDA_TRY(h, cudaMemcpyAsync(h.pinned + 44 + s, S.copy_off.as<int>() + S.n + 1, sizeof(int),
-                                      cudaMemcpyDeviceToHost, h.stream));
+    add(S.counted ? S.cell_start.as<int>() + S.ncells : S.copy_off.as<int>() + S.n, 32 + 2 * s);
+    add(S.real_scan.as<int>() + S.ncells, 33 + 2 * s);
+    if (S.counted) add(S.copy_off.as<int>() + S.n + 1, 44 + s);
   }
-  CLM_CUDA_TRY(h, cudaMemcpyAsync(h.pinned + 40, h.err.p, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
+  add(h.err.as<int>(), 40);
+  return t;
+}
+
+__global__ void k_totals(const __grid_constant__ Totals t) { copy_totals(t, threadIdx.x); }
+
+int enqueue_build_totals(Handle& h) {
+  k_totals<<<1, 32, 0, h.stream>>>(build_totals(h));
+  CLM_CUDA_TRY(h, cudaGetLastError());
+  h.launches++;
   return OK;
 }
 

@@ -190,6 +190,17 @@ constexpr size_t kResultBytes = 256 + 16 * 256 + 128;
 // Build (clm_build.cu)
 int scan_exclusive(Handle& h, const int* in, int* out, int64_t m, int* total, int depth = 0);
 template <class T> int build_set(Handle& h, int set, const Geometry<T>& g);
+// Words that a build leaves on the device for the host: the totals of every build not read back yet and the error
+// word, copied to the handle's pinned area by the kernel that ends the call (or by enqueue_build_totals).
+struct Totals {
+  const int* src[7];
+  int* dst[7];
+  int n;
+};
+__device__ __forceinline__ void copy_totals(const Totals& t, int k) {
+  if (k < t.n) *t.dst[k] = *t.src[k];
+}
+Totals build_totals(Handle& h);
 int enqueue_build_totals(Handle& h);
 int check_build_totals(Handle& h, bool* overflow);
 template <class T> int set_limits(Handle& h, T* lo, T* hi);

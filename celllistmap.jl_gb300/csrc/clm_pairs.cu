@@ -57,21 +57,23 @@ template <class T> __global__ void k_to_f32(const T* __restrict__ in, int64_t n,
   if (i < n) out[i] = (float)in[i];
 }
 
-// Fixed-order reductions of the per-block partials (deterministic results).
-__global__ void k_reduce_scalar(const double* __restrict__ pe, const unsigned long long* __restrict__ pc, int nb,
-                                double* __restrict__ out_e, unsigned long long* __restrict__ out_c) {
-  __shared__ double se[256];
-  __shared__ unsigned long long sc[256];
+// Fixed-order reductions of the per-block partials (deterministic results), by a block of 256 threads.
+constexpr int kReduce = 256;
+
+__device__ void reduce_scalar(const double* __restrict__ pe, const unsigned long long* __restrict__ pc, int nb,
+                              double* out_e, unsigned long long* out_c) {
+  __shared__ double se[kReduce];
+  __shared__ unsigned long long sc[kReduce];
   double e = 0;
   unsigned long long c = 0;
-  for (int b = threadIdx.x; b < nb; b += 256) {
+  for (int b = threadIdx.x; b < nb; b += kReduce) {
     e += pe[b];
     c += pc[b];
   }
   se[threadIdx.x] = e;
   sc[threadIdx.x] = c;
   __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
+  for (int s = kReduce / 2; s > 0; s >>= 1) {
     if ((int)threadIdx.x < s) {
       se[threadIdx.x] += se[threadIdx.x + s];
       sc[threadIdx.x] += sc[threadIdx.x + s];
@@ -84,53 +86,68 @@ __global__ void k_reduce_scalar(const double* __restrict__ pe, const unsigned lo
   }
 }
 
+// The smallest (d2, i, j): a total order, so the result does not depend on how it is split.  One thread walking
+// the 700 to 900 partials took 58 us.
 template <class T>
-__global__ void k_reduce_min(const T* __restrict__ pd, const int* __restrict__ pij, int nb, T* out_d, int* out_ij) {
-  if (threadIdx.x != 0) return;
+__device__ void reduce_min(const T* __restrict__ pd, const int* __restrict__ pij, int nb, T* out_d, int* out_ij) {
+  __shared__ T sd[kReduce];
+  __shared__ int si[kReduce], sj[kReduce];
   T bd = INFINITY;
   int bi = 0x7fffffff, bj = 0x7fffffff;
-  for (int b = 0; b < nb; b++) {
-    T d = pd[b];
-    int i = pij[2 * b], j = pij[2 * b + 1];
+  auto take = [&](T d, int i, int j) {
     if (d < bd || (d == bd && (i < bi || (i == bi && j < bj)))) {
       bd = d;
       bi = i;
       bj = j;
     }
+  };
+  for (int b = threadIdx.x; b < nb; b += kReduce) take(pd[b], pij[2 * b], pij[2 * b + 1]);
+  sd[threadIdx.x] = bd;
+  si[threadIdx.x] = bi;
+  sj[threadIdx.x] = bj;
+  __syncthreads();
+  for (int s = kReduce / 2; s > 0; s >>= 1) {
+    if ((int)threadIdx.x < s) {
+      take(sd[threadIdx.x + s], si[threadIdx.x + s], sj[threadIdx.x + s]);
+      sd[threadIdx.x] = bd;
+      si[threadIdx.x] = bi;
+      sj[threadIdx.x] = bj;
+    }
+    __syncthreads();
   }
-  *out_d = bd;
-  out_ij[0] = bi;
-  out_ij[1] = bj;
-}
-
-__global__ void k_reduce_vec(const double* __restrict__ pv, int nb, int k, double* __restrict__ out) {
-  const int c = threadIdx.x;
-  if (c >= k) return;
-  double s = 0;
-  for (int b = 0; b < nb; b++) s += pv[(int64_t)b * k + c];
-  out[c] = s;
-}
-
-__global__ void k_reduce_hist(const unsigned long long* __restrict__ pc, const double* __restrict__ ps, int nb,
-                              int nbins, unsigned long long* oc, double* os) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nbins) return;
-  unsigned long long c = 0;
-  double s = 0;
-  for (int k = 0; k < nb; k++) {
-    c += pc[(int64_t)k * nbins + b];
-    s += ps[(int64_t)k * nbins + b];
+  if (threadIdx.x == 0) {
+    *out_d = bd;
+    out_ij[0] = bi;
+    out_ij[1] = bj;
   }
-  oc[b] = c;
-  os[b] = s;
 }
 
-// forces: sums (rotated frame; 16-byte FP32 records or FP64 components) -> output dtype in the original
-// frame
+// Sum of column c of the nb x k partials, by one warp (in every lane).  One thread per column took 80 us for
+// the adjoint's 912 partials and 96 us for a histogram's.
+template <class V> __device__ __forceinline__ V column_sum(const V* __restrict__ p, int nb, int k, int c) {
+  V s = 0;
+  for (int b = threadIdx.x & 31; b < nb; b += 32) s += p[(int64_t)b * k + c];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+__global__ void __launch_bounds__(kReduce) k_reduce_scalar(const double* __restrict__ pe,
+                                                          const unsigned long long* __restrict__ pc, int nb,
+                                                          double* __restrict__ out_e, unsigned long long* __restrict__ out_c) {
+  reduce_scalar(pe, pc, nb, out_e, out_c);
+}
+template <class T>
+__global__ void __launch_bounds__(kReduce) k_reduce_min(const T* __restrict__ pd, const int* __restrict__ pij, int nb,
+                                                       T* out_d, int* out_ij) {
+  reduce_min(pd, pij, nb, out_d, out_ij);
+}
+
+// Force i from the sums (rotated frame; 16-byte FP32 records or FP64 components) in the output dtype and the
+// original frame.
 template <class T, int N, class FA>
-__global__ void k_forces_out(const FA* __restrict__ facc, int64_t n, DevGeom<T> g, int rotate, T* __restrict__ out) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+__device__ __forceinline__ void force_out(const FA* __restrict__ facc, int64_t i, const T (&Rinv)[3][3], int rotate,
+                                          T* __restrict__ out) {
   // FP32 sums are rotated in FP32 (the FP64 pipe is slow on this part); FP64 sums in FP64
   using R = typename std::conditional<std::is_same<FA, float4>::value, float, double>::type;
   R f[N];
@@ -149,7 +166,7 @@ __global__ void k_forces_out(const FA* __restrict__ facc, int64_t n, DevGeom<T> 
     for (int a = 0; a < N; a++) {
       R s = 0;
 #pragma unroll
-      for (int k = 0; k < N; k++) s += (R)g.Rinv[a][k] * f[k];
+      for (int k = 0; k < N; k++) s += (R)Rinv[a][k] * f[k];
       r[a] = s;
     }
 #pragma unroll
@@ -159,6 +176,71 @@ __global__ void k_forces_out(const FA* __restrict__ facc, int64_t n, DevGeom<T> 
   for (int d = 0; d < N; d++) out[i * N + d] = (T)f[d];
 }
 
+// What follows the pair kernel, in one launch: block 0 reduces the scalar partials (or the minimum) and copies the
+// totals of builds not read back yet, the next blocks sum the columns of a histogram or of the adjoint (one warp
+// each), the others convert the forces.  Results go straight to pinned host memory.  Before, a reduction, a
+// force kernel per set and four to seven copies of a few bytes: each a stream operation of 2 us on the host, of the
+// 110 us that a step of 32,000 particles takes.
+template <class T> struct FinishArgs {
+  int opk, nb;                    // operator kind, blocks of the pair kernel
+  const double* part_e;
+  const unsigned long long* part_c;
+  const T* part_min_d2;
+  const int* part_min_ij;
+  int nvec;                       // columns to sum: bins of a histogram, values of the adjoint
+  const unsigned long long* part_hc;
+  const double* part_hs;          // (the adjoint's values too)
+  unsigned long long* hc_out;     // histograms on the device: the caller's arrays
+  double* hs_out;
+  const unsigned long long* nl_count;
+  unsigned char* res;             // pinned: layout of kResultBytes
+  Totals totals;
+  const void* facc[2];            // force sums of sets x and y
+  T* fout[2];
+  int64_t fn[2];
+  unsigned fblocks0;              // blocks that convert the forces of set x
+  int f4, rotate;
+  T Rinv[3][3];
+};
+
+template <class T, int N> __global__ void __launch_bounds__(kReduce) k_finish(const __grid_constant__ FinishArgs<T> F) {
+  unsigned b = blockIdx.x;
+  if (b == 0) {
+    double* re = reinterpret_cast<double*>(F.res);
+    unsigned long long* rc = reinterpret_cast<unsigned long long*>(F.res + 8);
+    if (F.opk == OPK_SCALAR || F.opk == OPK_FORCES) reduce_scalar(F.part_e, F.part_c, F.nb, re, rc);
+    else if (F.opk == OPK_MIN)
+      reduce_min(F.part_min_d2, F.part_min_ij, F.nb, reinterpret_cast<T*>(F.res + 16), reinterpret_cast<int*>(F.res + 24));
+    else if (F.opk == OPK_NL && threadIdx.x == 0) *rc = *F.nl_count;
+    copy_totals(F.totals, threadIdx.x);
+    return;
+  }
+  b--;
+  const unsigned vblocks = (unsigned)(F.nvec + kReduce / 32 - 1) / (kReduce / 32);
+  if (b < vblocks) {
+    const int c = (int)(b * (kReduce / 32) + (threadIdx.x >> 5));
+    if (c >= F.nvec) return;
+    const double s = column_sum(F.part_hs, F.nb, F.nvec, c);
+    const bool lead = (threadIdx.x & 31) == 0;
+    if (F.opk == OPK_ADJ) {
+      if (lead) reinterpret_cast<double*>(F.res + 256 + 16 * 256)[c] = s;
+      return;
+    }
+    const unsigned long long n = column_sum(F.part_hc, F.nb, F.nvec, c);
+    if (lead) {
+      (F.hc_out ? F.hc_out : reinterpret_cast<unsigned long long*>(F.res + 256))[c] = n;
+      (F.hs_out ? F.hs_out : reinterpret_cast<double*>(F.res + 256 + 8 * 256))[c] = s;
+    }
+    return;
+  }
+  b -= vblocks;
+  const int set = b >= F.fblocks0;
+  if (set) b -= F.fblocks0;
+  const int64_t i = (int64_t)b * kReduce + threadIdx.x;
+  if (i >= F.fn[set]) return;
+  if (F.f4) force_out<T, N, float4>(static_cast<const float4*>(F.facc[set]), i, F.Rinv, F.rotate, F.fout[set]);
+  else force_out<T, N, double>(static_cast<const double*>(F.facc[set]), i, F.Rinv, F.rotate, F.fout[set]);
+}
 
 }  // namespace
 
@@ -381,7 +463,7 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
                             align(sizeof(T) * grid_want) + align(sizeof(int) * 2 * grid_want) +
                             (hist ? align(sizeof(unsigned long long) * grid_want * A.nbins) +
                                         align(sizeof(double) * grid_want * A.nbins) : 0) +
-                            align(sizeof(double) * kAdjVals * grid_want) + 4 * align(sizeof(double) * 512);
+                            align(sizeof(double) * kAdjVals * grid_want);
   if (!h.partial.reserve(part_bytes)) return ERR_NOMEM;
   char* pb = h.partial.as<char>();
   at = 0;
@@ -401,16 +483,8 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
   }
   A.part_v = (double*)(pb + at);
   at += align(sizeof(double) * kAdjVals * grid_want);
-  char* res = pb + at;  // final results
-  double* r_e = (double*)res;
-  unsigned long long* r_c = (unsigned long long*)(res + 8);
-  T* r_md = (T*)(res + 16);
-  int* r_mij = (int*)(res + 24);
-  unsigned long long* r_hc = (unsigned long long*)(res + 256);
-  double* r_hs = (double*)(res + 256 + 8 * 256);
   // outputs
   const bool forces = (opk == OPK_FORCES || opk == OPK_ADJ);
-  double* r_v = (double*)(res + 256 + 16 * 256);  // adjoint sums (kAdjVals)
   // forces are summed with atomics (FP32 pair values: 16-byte records; FP64: dim doubles per particle) in
   // the rotated frame and converted to the output after the map
   const bool f4 = !(std::is_same<T, double>::value && !A.split);
@@ -460,59 +534,60 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
       return ERR_CUDA;
     }
     h.launches++;
-    if (opk != OPK_NL) break;
-    unsigned long long n_pairs = 0;
-    CLM_CUDA_TRY(h, cudaMemcpyAsync(&n_pairs, A.nl_count, sizeof(n_pairs), cudaMemcpyDeviceToHost, h.stream));
-    CLM_CUDA_TRY(h, cudaStreamSynchronize(h.stream));
-    h.nl_n = (int64_t)n_pairs;
-    if ((int64_t)n_pairs <= h.nl_cap) break;
-    h.nl_cap = (int64_t)n_pairs + n_pairs / 16 + 1024;  // retry once with the exact size
-  }
-  if (opk == OPK_ADJ) {
-    k_reduce_vec<<<1, 32, 0, h.stream>>>(A.part_v, grid, kAdjVals, r_v);
-  } else if (opk == OPK_SCALAR || opk == OPK_FORCES) {
-    k_reduce_scalar<<<1, 256, 0, h.stream>>>(A.part_e, A.part_c, grid, r_e, r_c);
-  } else if (opk == OPK_MIN) {
-    k_reduce_min<T><<<1, 32, 0, h.stream>>>(A.part_min_d2, A.part_min_ij, grid, r_md, r_mij);
-  } else if (opk == OPK_HIST) {
-    k_reduce_hist<<<(A.nbins + 63) / 64, 64, 0, h.stream>>>(A.part_hc, A.part_hs, grid, A.nbins, r_hc, r_hs);
-  }
-  CLM_CUDA_TRY(h, cudaGetLastError());
-  if (opk != OPK_NL) h.launches++;
-  if (forces) {
-    const int rot = (g.kind == TRICLINIC) ? 1 : 0;
-    DevGeom<T>& dg = A.g;
-    h.launches += (nx && dst_x) + (ny && dst_y);
-    auto out = [&](int64_t cnt, int64_t first, T* dst) {
-      const unsigned blocks = (unsigned)((cnt + 255) / 256);
-      if (f4) {
-        if (N == 3) k_forces_out<T, 3, float4><<<blocks, 256, 0, h.stream>>>(A.f4x + first, cnt, dg, rot, dst);
-        else k_forces_out<T, 2, float4><<<blocks, 256, 0, h.stream>>>(A.f4x + first, cnt, dg, rot, dst);
-      } else {
-        if (N == 3) k_forces_out<T, 3, double><<<blocks, 256, 0, h.stream>>>(A.fx + first * N, cnt, dg, rot, dst);
-        else k_forces_out<T, 2, double><<<blocks, 256, 0, h.stream>>>(A.fx + first * N, cnt, dg, rot, dst);
+    FinishArgs<T> F;
+    std::memset(&F, 0, sizeof(F));
+    F.opk = opk;
+    F.nb = grid;
+    F.part_e = A.part_e;
+    F.part_c = A.part_c;
+    F.part_min_d2 = A.part_min_d2;
+    F.part_min_ij = A.part_min_ij;
+    F.nl_count = A.nl_count;
+    F.res = h.pres;
+    F.totals = build_totals(h);
+    if (opk == OPK_ADJ) {
+      F.nvec = kAdjVals;
+      F.part_hs = A.part_v;
+    } else if (hist) {
+      F.nvec = A.nbins;
+      F.part_hc = A.part_hc;
+      F.part_hs = A.part_hs;
+      if (O->out_on_device) {
+        F.hc_out = reinterpret_cast<unsigned long long*>(O->hist_count);
+        F.hs_out = O->hist_sum;
       }
-    };
-    if (nx && dst_x) out(nx, 0, dst_x);
-    if (ny && dst_y) out(ny, nx, dst_y);
+    }
+    unsigned blocks = 1 + (unsigned)(F.nvec + kReduce / 32 - 1) / (kReduce / 32);
+    if (forces) {
+      F.f4 = f4;
+      F.rotate = (g.kind == TRICLINIC) ? 1 : 0;
+      std::memcpy(F.Rinv, A.g.Rinv, sizeof(F.Rinv));
+      F.facc[0] = f4 ? (const void*)A.f4x : (const void*)A.fx;
+      F.facc[1] = f4 ? (const void*)A.f4y : (const void*)A.fy;
+      F.fout[0] = dst_x;
+      F.fout[1] = dst_y;
+      F.fn[0] = dst_x ? nx : 0;
+      F.fn[1] = dst_y ? ny : 0;
+      F.fblocks0 = (unsigned)((F.fn[0] + kReduce - 1) / kReduce);
+      blocks += F.fblocks0 + (unsigned)((F.fn[1] + kReduce - 1) / kReduce);
+    }
+    if (N == 3) k_finish<T, 3><<<blocks, kReduce, 0, h.stream>>>(F);
+    else k_finish<T, 2><<<blocks, kReduce, 0, h.stream>>>(F);
     CLM_CUDA_TRY(h, cudaGetLastError());
-    if (!O->out_on_device) {
+    h.launches++;
+    if (forces && !O->out_on_device) {
       if (O->forces_x && nx)
         CLM_CUDA_TRY(h, cudaMemcpyAsync(O->forces_x, dst_x, sizeof(T) * nx * N, cudaMemcpyDeviceToHost, h.stream));
       if (O->forces_y && ny)
         CLM_CUDA_TRY(h, cudaMemcpyAsync(O->forces_y, dst_y, sizeof(T) * ny * N, cudaMemcpyDeviceToHost, h.stream));
     }
+    CLM_CUDA_TRY(h, cudaStreamSynchronize(h.stream));
+    if (opk != OPK_NL) break;
+    std::memcpy(&h.nl_n, h.pres + 8, sizeof(h.nl_n));
+    if (h.nl_n <= h.nl_cap || attempt == 1) break;
+    h.nl_cap = h.nl_n + h.nl_n / 16 + 1024;  // retry once with the exact size
   }
-  // scalar results (and the totals of a build enqueued without synchronization), into pinned memory: only
-  // the part this operator wrote
   const char* hostres = reinterpret_cast<const char*>(h.pres);
-  const size_t res_bytes = (opk == OPK_HIST || opk == OPK_ADJ) ? kResultBytes : 32;
-  CLM_CUDA_TRY(h, cudaMemcpyAsync(h.pres, res, res_bytes, cudaMemcpyDeviceToHost, h.stream));
-  {
-    int st = enqueue_build_totals(h);
-    if (st) return st;
-  }
-  CLM_CUDA_TRY(h, cudaStreamSynchronize(h.stream));
   cudaEventElapsedTime(&h.map_ms, h.ev[2], h.ev[3]);
   if (h.build_timing_pending) {
     cudaEventElapsedTime(&h.build_ms, h.ev[0], h.ev[1]);
@@ -583,10 +658,7 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
     }
   }
   if (opk == OPK_HIST) {
-    if (O->out_on_device) {
-      CLM_CUDA_TRY(h, cudaMemcpyAsync(O->hist_count, r_hc, 8 * A.nbins, cudaMemcpyDeviceToDevice, h.stream));
-      CLM_CUDA_TRY(h, cudaMemcpyAsync(O->hist_sum, r_hs, 8 * A.nbins, cudaMemcpyDeviceToDevice, h.stream));
-    } else {
+    if (!O->out_on_device) {
       if (O->hist_count) std::memcpy(O->hist_count, hostres + 256, 8 * A.nbins);
       if (O->hist_sum) std::memcpy(O->hist_sum, hostres + 256 + 8 * 256, 8 * A.nbins);
     }
@@ -659,8 +731,8 @@ int run_pairs_scalar_scratch(Handle& h, const Geometry<T>& g, int op, const void
     return ERR_CUDA;
   }
   h.launches++;
-  if (opk == OPK_SCALAR) k_reduce_scalar<<<1, 256, 0, h.stream>>>(A.part_e, A.part_c, grid, r_e, r_c);
-  else k_reduce_min<T><<<1, 32, 0, h.stream>>>(A.part_min_d2, A.part_min_ij, grid, r_md, r_mij);
+  if (opk == OPK_SCALAR) k_reduce_scalar<<<1, kReduce, 0, h.stream>>>(A.part_e, A.part_c, grid, r_e, r_c);
+  else k_reduce_min<T><<<1, kReduce, 0, h.stream>>>(A.part_min_d2, A.part_min_ij, grid, r_md, r_mij);
   CLM_CUDA_TRY(h, cudaGetLastError());
   h.launches++;
   // results through the handle's pinned staging area (allocated when the handle was created)
