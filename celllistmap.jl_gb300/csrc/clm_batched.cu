@@ -241,6 +241,8 @@ template <class T> int enqueue_op(Handle& h, int slot, int op, const clm_op_para
   A.op = op;
   A.err = h.err.as<int>();
   A.cell_split = B.cell_split;
+  A.stage_split = 1;
+  A.stage = kStage;
   A.gtab = B.gtab.as<DevGeom<T>>();
   A.cell_sys = B.cell_sys.as<int>();
   A.cbase = B.cbase_d.as<int>();
@@ -287,19 +289,18 @@ template <class T> int enqueue_op(Handle& h, int slot, int op, const clm_op_para
     A.nl_cap = h.nl_cap;
     CLM_CUDA_TRY(h, cudaMemsetAsync(A.nl_count, 0, sizeof(unsigned long long), h.stream));
   }
-  // one resident wave (divided by the tuned factor)
-  int sms = 0, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // one resident wave (divided by the tuned factor): the resident blocks of the plain scalar kernel of the
+  // same shape
   const LaunchSel sel{N, opk, true, A.split != 0, true};
-  int grid = std::max(1, sms) * 64;
-  {
-    // resident blocks per SM of this instantiation: probe through the plain scalar kernel of the same
-    // shape, then apply the divisor
-    int per_sm = pairs_blocks_per_sm(LaunchSel{N, OPK_SCALAR, true, A.split != 0, false}, (const PairArgs<T>*)nullptr);
-    if (per_sm <= 0) per_sm = 1;
-    grid = std::max(1, per_sm * std::max(1, sms) / std::max(1, B.grid_div));
-  }
+  static const int sms = [] {
+    int n_sm = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    return std::max(1, n_sm);
+  }();
+  const int per_sm =
+      pairs_blocks_per_sm(LaunchSel{N, OPK_SCALAR, true, A.split != 0, false}, (const PairArgs<T>*)nullptr);
+  int grid = std::max(1, std::max(1, per_sm) * sms / std::max(1, B.grid_div));
   if (!h.capturing) cudaEventRecord(h.ev[2], h.stream);
   cudaError_t e = launch_pairs(sel, grid, h.stream, A);
   if (!h.capturing) cudaEventRecord(h.ev[3], h.stream);
@@ -368,7 +369,6 @@ template <class T> int finish_step(Handle& h, int nops, const int* ops, clm_batc
     return OK;
   }
   if (h.pinned[40] & DERR_CELL_RANGE) return fail(&h, ERR_INTERNAL, "batch consistency check failed");
-  if (h.pinned[40] & DERR_STAGE) return fail(&h, ERR_INTERNAL, "pair map: a staging wait for bulk copies timed out");
   int nl_slot = -1;
   for (int k = 0; k < nops; k++)
     if (ops[k] == CLM_OP_NL) nl_slot = k;

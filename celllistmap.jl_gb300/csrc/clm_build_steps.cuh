@@ -89,6 +89,7 @@ template <class T> void fill_devgeom(const Geometry<T>& g, int precision, DevGeo
   d.ncells = (int)g.ncells();
   for (int i = 0; i < 3; i++) {
     d.nc[i] = (int)g.nc[i];
+    if (i < 2) division_of(d.nc[i], &d.nc_mul[i], &d.nc_shift[i]);  // 2 lcell + 1 cells of margin: nc >= 2
     d.cbmin[i] = g.cbmin[i];
     d.cbmax[i] = g.cbmax[i];
     d.cs[i] = g.cs[i];

@@ -133,6 +133,8 @@ constexpr int kMaxDim = 3;
 template <class T> struct DevGeom {
   int dim, kind, lcell;
   int nc[3];
+  unsigned nc_mul[2];   // n / nc[k] = umulhi(n, nc_mul[k]) >> nc_shift[k] for 0 <= n < 2^31 (cart_of_fast)
+  int nc_shift[2];
   int ncells;
   T Min[3][3];    // input unit cell (wrap solve / product)
   T det_in;
@@ -375,6 +377,36 @@ __host__ __device__ __forceinline__ void cart_of(int li, const int* nc, int dim,
   }
 }
 
+// Multiplier and shift of n / d for 0 <= n < 2^31 and 2 <= d < 2^31 (Granlund and Montgomery's division by an
+// invariant integer): with s = ceil(log2 d) and m = ceil(2^(31+s) / d) < 2^32, the excess m d - 2^(31+s) is below
+// d <= 2^s, so floor(n m / 2^(31+s)) = floor(n / d) for every n < 2^31.
+inline void division_of(int d, unsigned* mul, int* shift) {
+  int s = 1;
+  while (((int64_t)1 << s) < d) s++;
+  *mul = (unsigned)((((uint64_t)1 << (31 + s)) + (uint64_t)d - 1) / (uint64_t)d);
+  *shift = s - 1;
+}
+__host__ __device__ __forceinline__ int div_fast(int n, unsigned mul, int shift) {
+#ifdef __CUDA_ARCH__
+  return (int)(__umulhi((unsigned)n, mul) >> shift);
+#else
+  return (int)((((uint64_t)(unsigned)n * mul) >> 32) >> shift);
+#endif
+}
+// cart_of with the geometry's division constants.
+template <int N, class T> __host__ __device__ __forceinline__ void cart_of_fast(const DevGeom<T>& g, int li, int* c) {
+  const int r = div_fast(li, g.nc_mul[0], g.nc_shift[0]);
+  c[0] = li - r * g.nc[0] + 1;
+  if (N == 3) {
+    c[2] = div_fast(r, g.nc_mul[1], g.nc_shift[1]);
+    c[1] = r - c[2] * g.nc[1] + 1;
+    c[2] += 1;
+  } else {
+    c[1] = r + 1;
+    c[2] = 1;
+  }
+}
+
 // cell_center (src/internals/Box.jl:517-525)
 template <class T, int N>
 __host__ __device__ __forceinline__ void cell_center(const DevGeom<T>& g, const int* c, T* ctr) {
@@ -535,10 +567,11 @@ template <class E> __host__ __device__ __forceinline__ int first_edge_at_or_abov
   return lo;
 }
 
-// FP32 distance rf within 2^-12 (relative) of one of the two edges around it (lo from
-// first_edge_at_or_above): the split form then decides the bin from the exact distance.
-__host__ __device__ __forceinline__ bool near_edge(const float* edges, int nbins, int lo, float rf) {
-  const float tol = rf * 2.44140625e-4f;
+// FP32 distance rf within 2^-12 (relative) plus `err` of one of the two edges around it (lo from
+// first_edge_at_or_above): the bin is then decided from the exact distance.  The split form only takes edges
+// that the relative window covers (err 0); the exact form adds the distance's absolute error and takes any.
+__host__ __device__ __forceinline__ bool near_edge(const float* edges, int nbins, int lo, float rf, float err = 0.f) {
+  const float tol = rf * 2.44140625e-4f + err;
   return (lo <= nbins && xabs(edges[lo] - rf) <= tol) || (lo >= 1 && xabs(edges[lo - 1] - rf) <= tol);
 }
 
@@ -549,7 +582,6 @@ enum DevError : int {
   DERR_COPY_OVERFLOW = 4,
   DERR_NL_OVERFLOW = 8,
   DERR_SCAN = 16,  // a single-pass scan gave up waiting for the prefix of an earlier tile
-  DERR_STAGE = 32, // the pair kernel gave up waiting for the bulk copies of a staging window
   DERR_TILE_OVERFLOW = 64,  // a tile of the counting build had more copies than its staging slots
 };
 

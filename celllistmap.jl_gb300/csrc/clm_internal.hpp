@@ -221,6 +221,5 @@ template <class T>
 int run_pairs_scalar_scratch(Handle& h, const Geometry<T>& g, int op, const void* params, void* outputs, void* scratch,
                              size_t scratch_bytes);
 int pairs_scalar_blocks_needed(Handle& h, int op);
-template <class T> int cell_split_for(const Handle& h, const Geometry<T>& g, int opk);
 
 }  // namespace clm

@@ -253,11 +253,10 @@ static double estimated_pairs(const Handle& h, double vol) {
   return std::max(0.0, nx * (double)h.sets[1].n * sph / vol);
 }
 
-// Parts per cell: cells holding many particles (large cutoff at high density) are split into parts
-// that take interleaved particle chunks, so that there are enough work items for every resident warp.
-// Each part keeps at least two chunks of 32 particles.
-template <class T> int cell_split_for(const Handle& h, const Geometry<T>& g, int opk) {
-  (void)opk;
+// Parts per cell of the round-based kernel: cells holding many particles (large cutoff at high density) are
+// split into parts that take interleaved particle chunks, each at least two chunks of 32 particles, until there
+// are two items per resident warp slot (24 warps per SM).
+template <class T> int round_split_for(const Handle& h, const Geometry<T>& g) {
   const double nx = (double)h.sets[0].n;
   double real_cells = 1.0;
   for (int i = 0; i < g.dim; i++) {
@@ -265,11 +264,46 @@ template <class T> int cell_split_for(const Handle& h, const Geometry<T>& g, int
     real_cells *= std::max(1.0, inner);
   }
   const double per_cell = nx / real_cells;
-  const double warps = 152.0 * 24.0 * 2.0;  // two items per resident warp slot (24 warps per SM)
+  const double warps = 152.0 * 24.0 * 2.0;
   int s = (int)std::ceil(warps / real_cells);
   s = std::min(s, (int)(per_cell / 64.0));
   s = std::max(1, std::min(s, 64));
   while (s > 1 && (double)g.ncells() * s >= 2147483647.0) s--;
+  return s;
+}
+
+// Work items of one map: every cell with real particles, in si parts of its particle chunks (of 32) times sj
+// parts of its candidate stages, until there are `kItems` of them (a few per resident warp, so that the last ones
+// do not leave the others waiting) or a part is one chunk against one stage.  When even that leaves warps
+// without an item, the stages are made smaller.
+struct ItemSplit {
+  int si, sj, stage;
+};
+template <class T> ItemSplit item_split_for(const Handle& h, const Geometry<T>& g) {
+  constexpr double kItems = 152.0 * 24.0 * 4.0;
+  const double nx = (double)h.sets[0].n, ny = (double)h.sets[h.nsets - 1].n;
+  double real_cells = 1.0, stencil = 1.0;
+  for (int i = 0; i < g.dim; i++) {
+    const double inner = (g.kind == NONPERIODIC) ? (double)g.nc[i] : (double)(g.nc[i] - 2 * g.lcell - 1);
+    real_cells *= std::max(1.0, inner);
+    stencil *= 2 * g.lcell + 1;
+  }
+  if (h.nsets == 1) stencil = (stencil + 1) / 2;
+  const double chunks = std::max(1.0, std::ceil(nx / real_cells / 32.0));
+  const double cands = ny / real_cells * stencil;
+  auto parts = [&](double have, double most) {
+    return (int)std::max(1.0, std::min({std::ceil(kItems / have), most, 4096.0}));
+  };
+  ItemSplit s;
+  s.si = parts(real_cells, chunks);
+  s.stage = kStage;
+  s.sj = parts(real_cells * s.si, std::ceil(cands / s.stage));
+  while (s.stage > 64 && real_cells * s.si * s.sj < 152.0 * 24.0) {
+    s.stage /= 2;
+    s.sj = parts(real_cells * s.si, std::ceil(cands / s.stage));
+  }
+  while (s.si > 1 && (double)g.ncells() * s.si * s.sj >= 2147483647.0) s.si--;
+  while (s.sj > 1 && (double)g.ncells() * s.si * s.sj >= 2147483647.0) s.sj--;
   return s;
 }
 
@@ -305,7 +339,12 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
   }
   A.op = op;
   A.err = h.err.as<int>();
-  A.cell_split = cell_split_for(h, g, opk);
+  const ItemSplit split = in_rounds(opk, sizeof(T) == 8, A.split != 0, false) ? ItemSplit{round_split_for(h, g), 1, kStage}
+                                                                             : item_split_for(h, g);
+  A.cell_split = split.si;
+  A.stage_split = split.sj;
+  A.stage = split.stage;
+  A.hist_err = (float)(split_distance_error(g) * 1.001);
   const LaunchSel sel{N, opk, A.self != 0, A.split != 0, false};
   const double c_default = (double)g.cutoff;
   {
@@ -456,7 +495,7 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
   // grid: static round-robin of real cells over warps (deterministic)
   // the number of real cells is only known on the device: size for all cells (one resident wave at most)
   const int grid_want =
-      (int)std::max<int64_t>(1, std::min<int64_t>((X.ncells * A.cell_split + kWarps - 1) / kWarps, 1 << 16));
+      (int)std::max<int64_t>(1, std::min<int64_t>((X.ncells * A.cell_split * A.stage_split + kWarps - 1) / kWarps, 1 << 16));
   int grid = grid_want;
   // partials
   const size_t part_bytes = align(sizeof(double) * grid_want) + align(sizeof(unsigned long long) * grid_want) +
@@ -603,10 +642,6 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
     h.last_error = "pair map consistency check failed (stencil cell outside the grid)";
     return ERR_INTERNAL;
   }
-  if (h.pinned[40] & DERR_STAGE) {
-    h.last_error = "pair map: a staging wait for bulk copies timed out";
-    return ERR_INTERNAL;
-  }
   std::memcpy(&O->scalar, hostres, 8);
   unsigned long long cnt;
   std::memcpy(&cnt, hostres + 8, 8);
@@ -700,6 +735,8 @@ int run_pairs_scalar_scratch(Handle& h, const Geometry<T>& g, int op, const void
   A.op = op;
   A.err = h.err.as<int>();
   A.cell_split = 1;
+  A.stage_split = 1;
+  A.stage = kStage;
   const LaunchSel sel{N, opk, A.self != 0, A.split != 0, false};
   {
     double pp[4] = {0, 0, 0, 0};
@@ -741,10 +778,6 @@ int run_pairs_scalar_scratch(Handle& h, const Geometry<T>& g, int op, const void
   CLM_CUDA_TRY(h, cudaStreamSynchronize(h.stream));
   if (h.pinned[4] & DERR_CELL_RANGE) {
     h.last_error = "pair map consistency check failed (stencil cell outside the grid)";
-    return ERR_INTERNAL;
-  }
-  if (h.pinned[4] & DERR_STAGE) {
-    h.last_error = "pair map: a staging wait for bulk copies timed out";
     return ERR_INTERNAL;
   }
   const char* hr = reinterpret_cast<const char*>(h.pinned + 8);

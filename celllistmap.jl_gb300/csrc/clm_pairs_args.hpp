@@ -13,6 +13,18 @@ namespace pk {
 
 constexpr int kWarps = 4;
 constexpr int kThreads = kWarps * 32;
+// Sizes of the pair kernel.  A stage holds at most kStage candidates in shared memory as planes of
+// coordinates and codes (kPad words of each plane per 32 candidates: 4 more than the candidates, so that the
+// lane groups of small chunks read different banks); kQueue hits fit the queue of a neighbour-list sweep (32
+// tests of every lane never give more); a warp's histogram bins hold at most kHistPairs pairs before they move
+// into the block's FP64 bins.
+constexpr int kStage = 256;
+constexpr int kPad = 36;
+constexpr int kPlane = kStage / 32 * kPad;
+constexpr int kQueue = 1024;
+constexpr int kHistPairs = 1024;
+// blocks per SM of the round-based adjoint: Float32 handles, the split form of Float64 handles
+constexpr int kAdjBlocks32 = 6, kAdjBlocks64 = 3;
 
 template <class T> struct SetView {
   const T* px;
@@ -37,6 +49,8 @@ template <class T> struct PairArgs {
   // operator parameters
   double p[4];
   float pf[4];  // the same in FP32 (set by set_params)
+  double ljd[5];  // LJ: sigma^2, eps c12, eps c6, 12 eps c12, 6 eps c6 (p = eps, sigma, c12, c6)
+  float ljf[5];
   int ntypes;
   const int* tx;
   const int* ty;
@@ -74,7 +88,10 @@ template <class T> struct PairArgs {
   double* part_hs;              // nbins per block
   double* part_v;               // kAdjVals per block (adjoint)
   // work decomposition and batches of independent systems
-  int cell_split;               // parts per cell: part p takes the particle chunks p, p + S, p + 2S, ...
+  int cell_split;               // parts of a cell's particles: part p takes the chunks p, p + S, p + 2S, ... of 32
+  int stage_split;              // parts of its candidates: part p takes the stages p, p + S, p + 2S, ...
+  int stage;                    // candidates per stage, at most kStage (a multiple of 32)
+  float hist_err;               // RHIST, Float64 exact: absolute error of the FP32 distance of cell offsets
   const DevGeom<T>* gtab;       // batch: geometry of each system
   const int* cell_sys;          // batch: system of each global cell
   const int* cbase;             // batch: first global cell of each system
@@ -86,9 +103,25 @@ template <class T> inline void set_params(PairArgs<T>& A, const double* p) {
     A.p[k] = p[k];
     A.pf[k] = (float)p[k];
   }
+  auto lj = [](auto* o, const auto* q) {
+    o[0] = q[1] * q[1];
+    o[1] = q[0] * q[2];
+    o[2] = q[0] * q[3];
+    o[3] = 12 * o[1];
+    o[4] = 6 * o[2];
+  };
+  lj(A.ljd, A.p);
+  lj(A.ljf, A.pf);
 }
 
 enum OpKind { OPK_NL = 0, OPK_SCALAR = 1, OPK_FORCES = 2, OPK_MIN = 3, OPK_HIST = 4, OPK_ADJ = 5 };
+// Maps of the round-based kernel (clm_pairs_rounds.cuh): FP32 sums (Float32 handles, the split form) that are
+// given out in FP64, whose last digits depend on the order of the additions: the adjoint, histograms, forces of
+// Float64 handles and the sums of batches.  k_pairs takes all other maps.
+constexpr bool in_rounds(int opk, bool f64, bool split, bool batch) {
+  return (!f64 || split) && (opk == OPK_ADJ || opk == OPK_HIST || (opk == OPK_FORCES && (f64 || batch)) ||
+                             (opk == OPK_SCALAR && batch));
+}
 constexpr int kAdjVals = 13;  // energy, virial (xx yy zz xy xz yz), dU/deps[3], dU/dsigma[3]
 
 // Dynamic shared memory of the radial-histogram kernel: block bins (FP64 sums, 64-bit counts), the bin
