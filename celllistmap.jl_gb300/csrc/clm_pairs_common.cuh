@@ -25,12 +25,14 @@ template <class T> __device__ __forceinline__ T pos_of(const SetView<T>& S, int 
 // Reciprocal and reciprocal square root for pair VALUES (energies, forces), which are checked against
 // tolerances, never used for pair membership or neighbour-list distances.
 //  FP32: hardware approximations (rcp.approx / rsqrt.approx, a couple of ulp).
-//  FP64: the hardware FP64 estimate y refined by the second-order terms of a series in its residual e,
-//        which cubes the relative error (from the estimate's ~2^-22 to far below FP64 rounding):
+//  FP64: the hardware FP64 estimate y (rcp / rsqrt.approx.ftz.f64: the upper word's value, relative error
+//        2^-20) refined by the second-order terms of a series in its residual e, which cubes the error to far
+//        below FP64 rounding:
 //        1/x = y / (1 - e) = y (1 + e + e^2 + ...) with e = 1 - x y;
 //        1/sqrt(x) = y (1 - e)^(-1/2) = y (1 + e/2 + 3e^2/8 + ...) with e = 1 - x y^2.
-//        Three and five FP64 instructions, where two Newton-Raphson steps take four and eight: GB300's FP64
-//        pipe takes 16 cycles per warp instruction and bounds the FP64 pair kernels.
+//        Three and five FP64 instructions: GB300's FP64 pipe takes 16 cycles per warp instruction and bounds the
+//        FP64 pair kernels.  rsqrt.approx.f64 without .ftz is a sequence of its own: refined, it took 11 FP64
+//        slots and was within 1.7e-16 of 1/sqrt(x); this takes 5.7 and is within 1.2e-16 (3e9 values).
 __device__ __forceinline__ float vrcp(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -46,21 +48,10 @@ __device__ __forceinline__ double vrcp(double x) {
 }
 __device__ __forceinline__ double vrsqrt(double x) {
   double y;
-  asm("rsqrt.approx.f64 %0, %1;" : "=d"(y) : "d"(x));
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = fma(-x, y * y, 1.0);
   const double p = fma(0.375, e, 0.5);  // 1/2 + 3e/8
   return fma(y * e, p, y);
-}
-
-// 1/sqrt(x) for the FP64 radial-histogram term: the hardware estimate refined by one Newton-Raphson step,
-// which squares its relative error (about 2^-23) to within ~1e-14 of 1/sqrt(x), far inside the 1e-10 to
-// which the per-bin sums are compared; each FP64 instruction saved frees the FP64 pipe that bounds the exact
-// histogram.
-__device__ __forceinline__ double vrsqrt_1nr(double x) {
-  double y;
-  asm("rsqrt.approx.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y * y, 1.0);
-  return fma(0.5 * y, e, y);
 }
 
 // a <= b and a < b for non-negative values (squared distances, the cutoff, +inf), decided on the bit

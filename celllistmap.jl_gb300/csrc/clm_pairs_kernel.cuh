@@ -813,12 +813,11 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
                           dot += (A.vxf[(int64_t)idx_i * N + d] - vy[(int64_t)idx_j * N + d]) * dv[d];
                         hv = dot * vrcp(rfl);
                       } else {
-                        // 1/r from the FP64 rsqrt estimate refined by one Newton step (vrsqrt_1nr)
                         const T* vy = CROSS ? A.vy : A.vx;
 #pragma unroll
                         for (int d = 0; d < N; d++)
                           dot += ((FA)A.vx[(int64_t)idx_i * N + d] - (FA)vy[(int64_t)idx_j * N + d]) * dv[d];
-                        hv = dot * (FA)vrsqrt_1nr((double)value_d2(q));
+                        hv = dot * (FA)vrsqrt((double)value_d2(q));
                       }
                       hb = b;
                     }
