@@ -72,7 +72,7 @@ template <class T> bool same_geometry(const Geometry<T>& a, const Geometry<T>& b
 
 template <class T> int build_all(Handle& h, bool sync) {
   if (!h.box_set) return fail(&h, ERR_STATE, "clm_set_box must be called before building");
-  for (int attempt = 0; attempt < 3; attempt++) {
+  for (int attempt = 0; attempt < 4; attempt++) {
     if (attempt > 0) CLM_CUDA_TRY(h, cudaMemsetAsync(h.err.p, 0, 64, h.stream));  // drop the overflow flag
     cudaEventRecord(h.ev[0], h.stream);
     bool rebuild_all = false;
@@ -288,7 +288,7 @@ int32_t clm_run(clm_handle h, int32_t op_id, const clm_op_params* params, clm_ou
   if (h->batch.on) return fail(h, ERR_STATE, "a batch handle takes clm_batched_set_systems / clm_batched_run");
   if (!h->box_set) return fail(h, ERR_STATE, "clm_set_box must be called before clm_run");
   drop_unchecked_builds(*h);
-  for (int attempt = 0; attempt < 3; attempt++) {
+  for (int attempt = 0; attempt < 4; attempt++) {
     bool need = false;
     for (int s = 0; s < h->nsets; s++) need = need || h->sets[s].dirty || !h->sets[s].built;
     cudaMemsetAsync(h->err.p, 0, 64, h->stream);

@@ -4,13 +4,14 @@
 // of add_particles! 940-950 and add_particle_to_celllist! 983-1057) and the
 // non-periodic build (src/internals/NonPeriodicCells.jl:93-251).
 //
-// One system (counting build, four launches after one memset):
-//   k_wrap_emit     wrap into the first cell (wrap_to_first, CellOperations.jl:91-94),
+// One system of at most 2^16 particles: k_build_small, the whole build in one cooperative launch.
+// One larger system (counting build, four launches after one memset):
+//   k_wrap_stage    wrap into the first cell (wrap_to_first, CellOperations.jl:91-94),
 //                   rotate, test the 3^N-1 translation images against the computing
-//                   box (replicate_particle!, Box.jl:556-566), scan the copies per
-//                   particle (decoupled look-back), write one (cell, particle<<5|image)
-//                   key/value per copy (particle_cell + real_particle_border_case), and
-//                   count the copies of every cell (atomic adds)
+//                   box (replicate_particle!, Box.jl:556-566), stage one (cell,
+//                   particle<<5|image) key/value per copy (particle_cell +
+//                   real_particle_border_case) in the tile's slots, and count the
+//                   copies of every cell (atomic adds)
 //   k_cell_scan     cell starts and the list of cells that contain real particles
 //   k_cell_scatter  copies to their cells' slots in arrival order (atomic cursors)
 //   k_rank_gather   each copy to its rank by value inside its cell (particle-index
@@ -614,6 +615,197 @@ __global__ void __launch_bounds__(kBlock) k_rank_gather(DevGeom<T> g, const T* _
   gather_at<T, N>(g, wrapped, t, p, k, (int)li, px, py, pz, off, xq, code, cell_flags, 0);
 }
 
+// ------------------------------------------------------------------ one system of few particles: one launch
+// The whole build in one cooperative kernel, for sets of at most kSmallParticles: the four kernels of the
+// counting build are each a few us of latency at these sizes.  Every warp wraps its particles (warps of
+// different blocks take neighbouring chunks, so that a thousand particles occupy 32 SMs and not four: a
+// warp's FP64 instruction holds its SM's pipe for 16 cycles), and every copy takes a slot of its cell's bucket
+// with one atomic.  After a barrier over the grid each block takes a range of cells: it sums the counts of the
+// cells before it, writes their starts and the real-cell list, and its warps rank the copies of a cell by
+// value (particle-index order) and gather them.  A cell with more than kBucket copies is flagged
+// (DERR_TILE_OVERFLOW) and the set is built by the other kernels from then on.
+constexpr int kSmallThreads = 512;
+constexpr int kBucket = 128;
+// Up to here the one launch is clearly the shorter build (GB300, Float32 / Float64 at liquid density: 4,000
+// particles 25 / 31 us against 37 / 43, 32,000 27 / 35 against 40 / 46, 64,000 30 / 40 against 39 / 50).  At 128,000
+// it still is, 40 / 57 against 46 / 65, but its blocks wait for a whole free device, which costs a program that
+// keeps other streams busy more than that; at 400,000 it is not (70 / 114 against 62 / 109).
+constexpr int64_t kSmallParticles = 1 << 16;
+constexpr int64_t kSmallCells = 1 << 15;
+constexpr double kSmallPerCell = 64.0;  // copies per cell expected at uniform density: half a bucket
+
+template <class T> struct SmallBuild {
+  DevGeom<T> g;
+  const T* x;
+  int n, ncells, cap;
+  T* wrapped;
+  uint32_t* bucket;   // kBucket values per cell
+  int* cf;            // {copies, holds a real particle} per cell, zero on entry
+  int* cf_next;       // the next build's, cleared here
+  unsigned* bar;      // {arrived, generation}
+  unsigned epoch;     // this launch's generation
+  int* cell_start;
+  int* cell_flags;
+  int* real_list;
+  int* n_real;
+  int* max_cell;
+  T* px;
+  T* py;
+  T* pz;
+  float4* off;
+  float4* xq;
+  int* code;
+  int* err;
+};
+
+template <class T, int N, int SH>
+__global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_constant__ SmallBuild<T> B) {
+  const DevGeom<T>& g = B.g;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kW = kSmallThreads / 32;
+  for (int c = blockIdx.x * kSmallThreads + threadIdx.x; c < 2 * B.ncells; c += gridDim.x * kSmallThreads) B.cf_next[c] = 0;
+  for (int i0 = (warp * gridDim.x + blockIdx.x) * 32; i0 < B.n; i0 += kW * gridDim.x * 32) {
+    const int i = i0 + lane;
+    if (i < B.n) {
+      T p[N];
+      uint32_t m = 0u;
+      int nc = 0;
+      if (!wrap_count_regs<T, N, SH>(g, B.x, i, p, m, nc)) atomicOr(B.err, DERR_NAN);
+#pragma unroll
+      for (int d = 0; d < N; d++) B.wrapped[(int64_t)i * N + d] = p[d];
+      for (int c = 0; c < nc; c++) {
+        int k = g.zero_code;
+        if (c > 0) {
+          k = lowest_bit(m);
+          m &= m - 1u;
+        }
+        const int key = copy_cell<T, N>(g, p, k, B.err);
+        const int slot = atomicAdd(&B.cf[2 * key], 1);
+        if (c == 0) B.cf[2 * key + 1] = 1;
+        if (slot < kBucket) B.bucket[(int64_t)key * kBucket + slot] = ((uint32_t)i << 5) | (uint32_t)k;
+        else atomicOr(B.err, DERR_TILE_OVERFLOW);
+      }
+    }
+  }
+  // ---- barrier over the grid (all blocks are resident: cooperative launch).  The last block to arrive opens it.
+  __shared__ int s_ok;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_ok = 1;
+    if (atomicAdd(&B.bar[0], 1u) == gridDim.x - 1) {
+      B.bar[0] = 0u;
+      __threadfence();
+      atomicExch(&B.bar[1], B.epoch);
+    } else {
+      int spins = 0;
+      while (*(volatile unsigned*)&B.bar[1] != B.epoch) {
+        if (++spins > kScanSpinLimit) {
+          atomicOr(B.err, DERR_SCAN);
+          s_ok = 0;
+          break;
+        }
+        __nanosleep(20);
+      }
+    }
+    __threadfence();
+  }
+  __syncthreads();
+  if (!s_ok) return;
+  // ---- this block's cells; what other blocks wrote is read past L1 (__ldcg)
+  const int per = (B.ncells + gridDim.x - 1) / gridDim.x;
+  const int c0 = min(B.ncells, (int)blockIdx.x * per), c1 = min(B.ncells, c0 + per);
+  __shared__ int s_sum[2][kW];
+  __shared__ int s_base[2];
+  __shared__ int wsum_c[kW + 1], wsum_f[kW + 1];
+  const int2* cf2 = reinterpret_cast<const int2*>(B.cf);
+  {
+    int sc = 0, sf = 0;
+    for (int c = threadIdx.x; c < c0; c += kSmallThreads) {
+      const int2 v = __ldcg(cf2 + c);
+      sc += v.x;
+      sf += v.y;
+    }
+    sc = __reduce_add_sync(0xffffffffu, sc);
+    sf = __reduce_add_sync(0xffffffffu, sf);
+    if (lane == 0) {
+      s_sum[0][warp] = sc;
+      s_sum[1][warp] = sf;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+      int t = 0;
+      for (int k = 0; k < kW; k++) t += s_sum[threadIdx.x][k];
+      s_base[threadIdx.x] = t;
+    }
+    __syncthreads();
+  }
+  const bool skip = (__ldcg(B.err) & (DERR_TILE_OVERFLOW | DERR_NAN)) != 0;  // the cell list is not used
+  for (int cb = c0; cb < c1; cb += kSmallThreads) {  // 512 cells at a time
+    const int c = cb + threadIdx.x;
+    int2 v = make_int2(0, 0);
+    if (c < c1) v = __ldcg(cf2 + c);
+    int vc[1] = {v.x}, vf[1] = {v.y}, off_c, off_f;
+    const int agg_c = block_scan<1, kSmallThreads>(vc, off_c, wsum_c);
+    const int agg_f = block_scan<1, kSmallThreads>(vf, off_f, wsum_f);
+    const int start = s_base[0] + off_c + vc[0], fpos = s_base[1] + off_f + vf[0];
+    if (c < c1) {
+      B.cell_start[c] = start;
+      B.cell_flags[c] = v.y;
+      if (v.y) B.real_list[fpos] = c;
+      if (c == B.ncells - 1) {
+        B.cell_start[B.ncells] = start + v.x;
+        *B.n_real = fpos + v.y;
+        *B.max_cell = 0;
+      }
+      if (start + v.x > B.cap) atomicOr(B.err, DERR_COPY_OVERFLOW);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_base[0] += agg_c;
+      s_base[1] += agg_f;
+    }
+    __syncthreads();
+  }
+  if (skip) return;
+  __syncthreads();  // the starts written above are read below by the block that wrote them
+  for (int c = c0 + warp; c < c1; c += kW) {
+    const int s = B.cell_start[c];
+    const int cnt = __ldcg(&B.cf[2 * c]);
+    if (cnt == 0 || s + cnt > B.cap) continue;
+    uint32_t v[kBucket / 32];
+    int r[kBucket / 32];
+#pragma unroll
+    for (int q = 0; q < kBucket / 32; q++) {
+      v[q] = (32 * q + lane < cnt) ? __ldcg(&B.bucket[(int64_t)c * kBucket + 32 * q + lane]) : 0xffffffffu;
+      r[q] = 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kBucket / 32; q++) {
+      const int e = min(32, cnt - 32 * q);
+      for (int k = 0; k < e; k++) {
+        const uint32_t u = __shfl_sync(0xffffffffu, v[q], k);
+#pragma unroll
+        for (int z = 0; z < kBucket / 32; z++) r[z] += (u < v[z]) ? 1 : 0;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kBucket / 32; q++) {
+      if (32 * q + lane < cnt) {
+        const int p = (int)(v[q] >> 5), k = (int)(v[q] & 31u);
+        if (p >= B.n || k >= g.nimg || r[q] >= cnt) {
+          atomicOr(B.err, DERR_CELL_RANGE);
+          continue;
+        }
+        T w[N];
+#pragma unroll
+        for (int d = 0; d < N; d++) w[d] = __ldcg(&B.wrapped[(int64_t)p * N + d]);
+        gather_copy<T, N>(g, w, s + r[q], p, k, c, B.px, B.py, B.pz, B.off, B.xq, B.code);
+      }
+    }
+  }
+}
+
 // Crowded cells (radix path of one system): the cells with real particles, in linear order, in one pass:
 // each tile scans its cells' flags, takes its first slot by decoupled look-back, and lists its flagged
 // cells; the last tile writes their number.
@@ -839,15 +1031,90 @@ template <class T> int set_limits(Handle& h, T* lo, T* hi) {
 // uniform-density estimate (computing-box volume / unit-cell volume), with a margin.  The build never
 // waits for the device: if the copies exceed the capacity, the key kernel flags it, the result is discarded at
 // the next host synchronization and the build is repeated with the exact size.
-template <class T> int64_t copy_capacity(const SetData& S, const Geometry<T>& g) {
-  const int64_t n = S.n;
-  if (g.kind == NONPERIODIC) return n + 64;
+template <class T> double copies_expected(const SetData& S, const Geometry<T>& g) {
+  if (g.kind == NONPERIODIC) return (double)S.n;
   double vbox = 1.0;
   for (int i = 0; i < g.dim; i++) vbox *= (double)g.cbmax[i] - (double)g.cbmin[i];
   const double vcell = std::fabs((double)g.det_in);
-  double est = (vcell > 0) ? (double)n * vbox / vcell : 27.0 * (double)n;
-  est = std::min(est * 1.15 + 4096.0, 27.0 * (double)n + 64.0);
+  return (vcell > 0) ? (double)S.n * vbox / vcell : 27.0 * (double)S.n;
+}
+template <class T> int64_t copy_capacity(const SetData& S, const Geometry<T>& g) {
+  const int64_t n = S.n;
+  if (g.kind == NONPERIODIC) return n + 64;
+  const double est = std::min(copies_expected(S, g) * 1.15 + 4096.0, 27.0 * (double)n + 64.0);
   return std::max<int64_t>(std::max<int64_t>(S.copy_cap, (int64_t)est), n + 64);
+}
+
+// One system of few particles: k_build_small.  `launched` says whether it took the build (a device that cannot hold
+// the grid at once leaves it to the counting build).
+template <class T>
+int build_small(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, int64_t ncells, int64_t cap, bool* launched) {
+  *launched = false;
+  using Kernel = void (*)(const SmallBuild<T>);
+  Kernel k = (N == 3) ? (Kernel)k_build_small<T, 3, kShapeGeneral> : (Kernel)k_build_small<T, 2, kShapeGeneral>;
+  if constexpr (std::is_same<T, double>::value) {
+    if (N == 3 && dg.shape == kShapeDiag) k = k_build_small<T, 3, kShapeDiag>;
+    else if (N == 3 && dg.shape == kShapeUpper) k = k_build_small<T, 3, kShapeUpper>;
+  }
+  static const int sms = [] {
+    int v = 0, dev = 0, coop = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    return coop ? v : 0;
+  }();
+  if (sms <= 0) return OK;
+  // the counters of this build and the next, the barrier, and the buckets
+  const size_t words = 4 * (size_t)ncells + 2;
+  const void* at = S.small_buf.p;
+  if (!S.small_buf.reserve(sizeof(int) * (words + kBucket * (size_t)ncells)) ||
+      !S.wrapped.reserve(sizeof(T) * N * n) || !S.px.reserve(sizeof(T) * cap) || !S.py.reserve(sizeof(T) * cap) ||
+      !S.pz.reserve(sizeof(T) * cap) ||
+      !S.off.reserve(std::is_same<T, float>::value ? 16 : sizeof(float4) * cap) || !S.code.reserve(sizeof(int) * cap) ||
+      !S.xq.reserve(std::is_same<T, float>::value ? sizeof(float4) * cap : 16))
+    return ERR_NOMEM;
+  if (S.small_cells != ncells || S.small_buf.p != at) {
+    S.small_cells = 0;
+    CLM_CUDA_TRY(h, cudaMemsetAsync(S.small_buf.p, 0, sizeof(int) * words, h.stream));
+    S.small_cells = ncells;
+    S.small_epoch = 0;
+  }
+  S.small_epoch++;
+  SmallBuild<T> B;
+  B.g = dg;
+  B.x = S.x.as<T>();
+  B.n = (int)n;
+  B.ncells = (int)ncells;
+  B.cap = (int)cap;
+  B.wrapped = S.wrapped.as<T>();
+  B.bucket = S.small_buf.as<uint32_t>() + words;
+  B.cf = S.small_buf.as<int>() + ((S.small_epoch & 1) ? 2 * ncells : 0);
+  B.cf_next = S.small_buf.as<int>() + ((S.small_epoch & 1) ? 0 : 2 * ncells);
+  B.bar = reinterpret_cast<unsigned*>(S.small_buf.as<int>() + 4 * ncells);
+  B.epoch = S.small_epoch;
+  B.cell_start = S.cell_start.as<int>();
+  B.cell_flags = S.cell_flags.as<int>();
+  B.real_list = S.real_list.as<int>();
+  B.n_real = S.real_scan.as<int>() + ncells;
+  B.max_cell = S.copy_off.as<int>() + n + 1;
+  B.px = S.px.as<T>();
+  B.py = S.py.as<T>();
+  B.pz = S.pz.as<T>();
+  B.off = S.off.as<float4>();
+  B.xq = S.xq.as<float4>();
+  B.code = S.code.as<int>();
+  B.err = h.err.as<int>();
+  void* args[] = {&B};
+  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k, dim3((unsigned)sms), dim3(kSmallThreads), args, 0, h.stream);
+  if (e != cudaSuccess) S.small_cells = 0;
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    return OK;
+  }
+  CLM_CUDA_TRY(h, e);
+  h.launches++;
+  *launched = true;
+  return OK;
 }
 
 // One system: the counting build.  One zeroed region holds the look-back words of the cell scan and the
@@ -999,6 +1266,13 @@ template <class T> int build_set(Handle& h, int set, const Geometry<T>& g) {
   // sort's cost does not depend on it.  Either gives the same cell list.
   const bool crowded = !batch && (S.prefer_radix || (double)cap > kCountingMaxPerCell * (double)ncells);
   S.counted = !batch && !crowded;
+  S.small = false;
+  if (!batch && !S.prefer_radix && !S.small_off && n <= kSmallParticles && ncells <= kSmallCells &&
+      copies_expected(S, g) <= kSmallPerCell * (double)ncells) {
+    const int st = build_small<T>(h, S, dg, N, n, ncells, cap, &S.small);
+    if (S.small) S.counted = true;
+    if (st || S.small) return st;
+  }
   if (S.counted) return build_counting<T>(h, S, dg, N, n, ncells, cap);
   // the radix path's gather sets the real flags of the cells it fills
   CLM_CUDA_TRY(h, cudaMemsetAsync(S.cell_flags.p, 0, sizeof(int) * (ncells + 1), h.stream));
@@ -1186,7 +1460,12 @@ int check_build_totals(Handle& h, bool* overflow) {
     S.n_copies = h.pinned[32 + 2 * s];
     S.n_real_cells = h.pinned[33 + 2 * s];
     if (S.counted && h.pinned[44 + s] > kRadixAbovePerCell) S.prefer_radix = true;
-    if (S.counted && (errw & DERR_TILE_OVERFLOW)) {
+    if (S.small && (errw & DERR_TILE_OVERFLOW)) {
+      // a cell had more copies than its bucket: the counting build (or radix, when it finds the cell crowded)
+      S.small_off = true;
+      S.dirty = true;
+      *overflow = true;
+    } else if (S.counted && (errw & DERR_TILE_OVERFLOW)) {
       // a tile had more copies than its staging slots: more slots per particle, and build again
       S.tile_mult = std::min(27, 2 * S.tile_mult);
       S.dirty = true;
@@ -1202,6 +1481,7 @@ int check_build_totals(Handle& h, bool* overflow) {
     }
   }
   if (errw & DERR_SCAN) {
+    for (int s = 0; s < h.nsets; s++) h.sets[s].small_cells = 0;  // a barrier left half open is cleared
     h.last_error = "cell-list build: a scan tile gave up waiting for an earlier tile";
     return ERR_INTERNAL;
   }

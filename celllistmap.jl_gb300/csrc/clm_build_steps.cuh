@@ -435,18 +435,15 @@ __host__ __device__ __forceinline__ void cell_starts_at(const uint32_t* __restri
   for (int c = lo; c <= hi && c <= ncells; c++) cell_start[c] = t;
 }
 
-// Copy t of the sorted list: particle p, image k, in the cell `li` (local index of its system).
+// Copy t of the cell list: image k of particle p, at wrapped position w, in the cell `li` (local index of its
+// system).
 template <class T, int N>
-__host__ __device__ __forceinline__ void gather_at(const DevGeom<T>& g, const T* __restrict__ wrapped, int t, int p, int k,
-                                          int li, T* __restrict__ px, T* __restrict__ py, T* __restrict__ pz,
-                                          float4* __restrict__ off, float4* __restrict__ xq,
-                                          int* __restrict__ code, int* __restrict__ cell_flags, int cb) {
+__host__ __device__ __forceinline__ void gather_copy(const DevGeom<T>& g, const T* w, int t, int p, int k, int li,
+                                            T* __restrict__ px, T* __restrict__ py, T* __restrict__ pz,
+                                            float4* __restrict__ off, float4* __restrict__ xq, int* __restrict__ code) {
   T q[N];
 #pragma unroll
-  for (int d = 0; d < N; d++) {
-    T w = wrapped[(int64_t)p * N + d];
-    q[d] = (k == g.zero_code) ? w : xadd(w, g.shift[k][d]);
-  }
+  for (int d = 0; d < N; d++) q[d] = (k == g.zero_code) ? w[d] : xadd(w[d], g.shift[k][d]);
   const int pc = (k == g.zero_code) ? p : -(p + 1);
   px[t] = q[0];
   py[t] = q[1];
@@ -456,7 +453,7 @@ __host__ __device__ __forceinline__ void gather_at(const DevGeom<T>& g, const T*
     xq[t] = make_float4((float)q[0], (float)q[1], N == 3 ? (float)q[N - 1] : 0.f, bits_as_float(pc));
   } else {
     int c[3];
-    cart_of(li, g.nc, N, c);
+    cart_of_fast<N>(g, li, c);
     float o[3] = {0.f, 0.f, 0.f};
 #pragma unroll
     for (int d = 0; d < N; d++) {
@@ -469,6 +466,17 @@ __host__ __device__ __forceinline__ void gather_at(const DevGeom<T>& g, const T*
     off[t] = make_float4(o[0], o[1], o[2], bits_as_float(pc));
   }
   code[t] = pc;
+}
+// The same from the array of wrapped positions; a real copy marks its cell.
+template <class T, int N>
+__host__ __device__ __forceinline__ void gather_at(const DevGeom<T>& g, const T* __restrict__ wrapped, int t, int p, int k,
+                                          int li, T* __restrict__ px, T* __restrict__ py, T* __restrict__ pz,
+                                          float4* __restrict__ off, float4* __restrict__ xq,
+                                          int* __restrict__ code, int* __restrict__ cell_flags, int cb) {
+  T w[N];
+#pragma unroll
+  for (int d = 0; d < N; d++) w[d] = wrapped[(int64_t)p * N + d];
+  gather_copy<T, N>(g, w, t, p, k, li, px, py, pz, off, xq, code);
   if (k == g.zero_code) cell_flags[cb + li] = 1;  // the cell holds a real particle
 }
 

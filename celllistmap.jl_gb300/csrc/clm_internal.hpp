@@ -89,6 +89,12 @@ struct SetData {
   int tile_mult = 0;         // counting build: staging slots per particle of a tile (0: from the estimate)
   int64_t n_cells_with_particles = 0;
   int64_t ncells = 0;
+  // build of a few particles in one launch (k_build_small)
+  DevBuf small_buf;          // two sets of per-cell counters, the grid barrier, each cell's copies in arrival order
+  int64_t small_cells = 0;   // cells that it is laid out and cleared for (0: none)
+  unsigned small_epoch = 0;  // launches since then
+  bool small = false;        // the last build was one
+  bool small_off = false;    // one met a cell with more copies than a bucket holds
 };
 
 struct ScanTemp {
