@@ -274,8 +274,10 @@ template <class T> int round_split_for(const Handle& h, const Geometry<T>& g) {
 
 // Work items of one map: every cell with real particles, in si parts of its particle chunks (of 32) times sj
 // parts of its candidate stages, until there are `kItems` of them (a few per resident warp, so that the last ones
-// do not leave the others waiting) or a part is one chunk against one stage.  When even that leaves warps
-// without an item, the stages are made smaller.
+// do not leave the others waiting) or a part is one chunk against one stage.  When even that leaves fewer
+// than 12 warps per SM with an item, the stages are made smaller.  Each part reads the cell's table and its
+// particles again, so not up to the full 24: a map of 32k Lennard-Jones particles takes 26.6 us with the line at 8
+// or 12 warps and 30.7 us at 24, the closest pair of 1501 and 4507 points 26.4 us at 8 and 24.6 us at 12 or 24.
 struct ItemSplit {
   int si, sj, stage;
 };
@@ -298,7 +300,7 @@ template <class T> ItemSplit item_split_for(const Handle& h, const Geometry<T>& 
   s.si = parts(real_cells, chunks);
   s.stage = kStage;
   s.sj = parts(real_cells * s.si, std::ceil(cands / s.stage));
-  while (s.stage > 64 && real_cells * s.si * s.sj < 152.0 * 24.0) {
+  while (s.stage > 64 && real_cells * s.si * s.sj < 152.0 * 12.0) {
     s.stage /= 2;
     s.sj = parts(real_cells * s.si, std::ceil(cands / s.stage));
   }
