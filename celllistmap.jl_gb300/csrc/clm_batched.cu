@@ -89,7 +89,7 @@ template <class T> int batch_tables(Handle& h) {
   std::vector<DevGeom<T>> tab((size_t)nsys);
   B.cbase.assign((size_t)nsys + 1, 0);
   B.status.assign((size_t)nsys, OK);
-  B.copies_est = B.pairs_est = B.real_cells = 0;
+  B.copies_est = B.cell_est = B.pairs_est = B.real_cells = 0;
   const double pi = 3.14159265358979323846;
   const double sph = (N == 2 ? pi : 4.0 * pi / 3.0) * std::pow(B.cutoff, N);
   bool have = false;
@@ -112,13 +112,15 @@ template <class T> int batch_tables(Handle& h) {
     if (total >= ((int64_t)1 << 30)) return fail(&h, ERR_ARG, "too many cells in the batch (reduce lcell)");
     B.cbase[(size_t)s + 1] = (int)total;
     const double ns = (double)(B.offsets[(size_t)s + 1] - B.offsets[(size_t)s]);
-    double vbox = 1.0, real = 1.0;
+    double vbox = 1.0, real = 1.0, in_cell = ns;
     for (int i = 0; i < N; i++) {
       vbox *= (double)g.cbmax[i] - (double)g.cbmin[i];
       real *= std::max(1.0, (double)(g.nc[i] - 2 * g.lcell - 1));
+      in_cell *= (double)g.cs[i];
     }
     const double vcell = std::fabs((double)g.det_in);
     B.copies_est += (vcell > 0) ? ns * vbox / vcell : 27.0 * ns;
+    if (vcell > 0) B.cell_est = std::max(B.cell_est, in_cell / vcell);
     B.pairs_est += (vcell > 0) ? ns * (ns - 1) / 2 * sph / vcell : 0.0;
     B.real_cells += real;
     if (!have) {

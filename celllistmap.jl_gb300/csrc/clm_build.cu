@@ -470,11 +470,12 @@ __global__ void __launch_bounds__(WE_BLOCK) k_wrap_stage(DevGeom<T> g, const T* 
 // cells' copy counts and real flags, takes both prefixes by decoupled look-back (warp 0 the counts, warp 1
 // the flags; one ticket orders the tiles of both), and writes cell_start, the real flags the pair kernel
 // reads, and the real cells in linear order.  The last tile closes cell_start and writes the number of
-// real cells.  Each cell's counters are cleared after reading: they are the scatter's cursors next.
+// real cells (batches: and the number of real cells before each, real_scan).  Each cell's counters are cleared after
+// reading: they are the scatter's cursors next, or the next build's counters.
 __global__ void __launch_bounds__(kBlock) k_cell_scan(int* __restrict__ cell_cf, int ncells,
                                                       int* __restrict__ cell_start, int* __restrict__ cell_flags,
-                                                      int* __restrict__ real_list, int* __restrict__ n_real,
-                                                      int* __restrict__ max_cell,
+                                                      int* __restrict__ real_list, int* __restrict__ real_scan,
+                                                      int* __restrict__ n_real, int* __restrict__ max_cell,
                                                       unsigned long long* __restrict__ status_c,
                                                       unsigned long long* __restrict__ status_f,
                                                       unsigned* __restrict__ ticket, int ntiles,
@@ -531,6 +532,7 @@ __global__ void __launch_bounds__(kBlock) k_cell_scan(int* __restrict__ cell_cf,
       cell_start[c] = vc[k] + off_c;
       cell_flags[c] = f[k];
       if (f[k]) real_list[vf[k] + off_f] = c;
+      if (real_scan) real_scan[c] = vf[k] + off_f;
     }
   }
 }
@@ -615,6 +617,199 @@ __global__ void __launch_bounds__(kBlock) k_rank_gather(DevGeom<T> g, const T* _
   gather_at<T, N>(g, wrapped, t, p, k, (int)li, px, py, pz, off, xq, code, cell_flags, 0);
 }
 
+// ------------------------------------------------------------------ buckets: wrap and place, gather
+// The builds that place every copy once: each cell has `slots` places, and a copy takes the next one of its cell with
+// one atomic when its key is known, so no list of keys is written, read back and scattered.  A cell with more copies
+// than places sets DERR_TILE_OVERFLOW (the build is repeated with more places, or by the counting build).
+//
+// A warp's copies are shared out evenly over its block before their cells are computed: most particles have one
+// copy, a few have seven, and lanes that walked their own would leave the others idle (and in Float64 hold the FP64
+// pipe, 16 cycles per warp instruction, for each round).
+template <class T> struct PlaceArgs {
+  DevGeom<T> g;
+  const DevGeom<T>* gtab;  // batches: geometry per system, system of each particle, first cell of each system
+  const int* psys;
+  const int* cbase;
+  int* sys_err;
+  const T* x;
+  int n;
+  T* wrapped;
+  uint32_t* bucket;  // `slots` values per cell
+  int slots;
+  int* cf;           // {copies, holds a real particle} per cell, zero before the build
+  int* err;
+};
+template <class T, int N, int NT> struct PlaceShared {
+  T pos[NT][N];
+  T shift[27][3];
+  int sys[NT];
+  int wsum[NT / 32 + 1];
+  uint16_t list[NT * (N == 3 ? 27 : 9)];  // copies of the block's particles: thread << 5 | image code
+};
+template <class T> __device__ __forceinline__ void load_shift(const DevGeom<T>& g, T (*shift)[3]) {
+  for (int t = threadIdx.x; t < 27 * 3; t += blockDim.x) shift[t / 3][t % 3] = g.shift[t / 3][t % 3];
+}
+// Particles first + warp * stride + lane of one block of NT threads (at most 2048).  One system: sm.shift holds the
+// geometry's shifts (visible after the scan's barriers).
+template <class T, int N, int SH, int NT, bool BATCH>
+__device__ __forceinline__ void place_copies(const PlaceArgs<T>& P, int first, int stride, PlaceShared<T, N, NT>& sm) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = first + warp * stride + lane;
+  T p[N];
+  uint32_t m = 0u;
+  int v[1] = {0};
+  if (i < P.n) {
+    bool ok = true;
+    if constexpr (BATCH) {
+      const int s = P.psys[i];
+      sm.sys[threadIdx.x] = s;
+      const DevGeom<T>& g = P.gtab[s];
+      if (g.ncells == 0) {  // a system that failed the unit-cell check has no copies
+#pragma unroll
+        for (int d = 0; d < N; d++) p[d] = T(0);
+      } else {
+        ok = wrap_count_regs<T, N, SH>(g, P.x, i, p, m, v[0]);
+        if (!ok) atomicOr(&P.sys_err[s], DERR_NAN);
+      }
+    } else {
+      ok = wrap_count_regs<T, N, SH>(P.g, P.x, i, p, m, v[0]);
+      if (!ok) atomicOr(P.err, DERR_NAN);
+    }
+#pragma unroll
+    for (int d = 0; d < N; d++) {
+      P.wrapped[(int64_t)i * N + d] = p[d];
+      sm.pos[threadIdx.x][d] = p[d];
+    }
+  }
+  const int nc = v[0];
+  int off = 0;
+  const int agg = block_scan<1, NT>(v, off, sm.wsum);
+  if (nc > 0) {
+    const int zero = BATCH ? (N == 3 ? 13 : 4) : P.g.zero_code;
+    uint16_t* at = sm.list + off + v[0];
+    *at++ = (uint16_t)(threadIdx.x << 5 | zero);
+    while (m) {
+      *at++ = (uint16_t)(threadIdx.x << 5 | lowest_bit(m));
+      m &= m - 1u;
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < agg; e += NT) {
+    const int w = sm.list[e], t = w >> 5, k = w & 31;
+    T q[N];
+#pragma unroll
+    for (int d = 0; d < N; d++) q[d] = sm.pos[t][d];
+    int key;
+    bool real;
+    if constexpr (BATCH) {
+      const DevGeom<T>& g = P.gtab[sm.sys[t]];
+      key = P.cbase[sm.sys[t]] + copy_cell<T, N>(g, q, k, P.err);
+      real = k == (N == 3 ? 13 : 4);
+    } else {
+      key = copy_cell<T, N>(P.g, sm.shift, q, k, P.err);
+      real = k == P.g.zero_code;
+    }
+    const int slot = atomicAdd(&P.cf[2 * (int64_t)key], 1);
+    if (real) P.cf[2 * (int64_t)key + 1] = 1;
+    const int at = first + (t >> 5) * stride + (t & 31);
+    if (slot < P.slots) P.bucket[(int64_t)key * P.slots + slot] = ((uint32_t)at << 5) | (uint32_t)k;
+    else atomicOr(P.err, DERR_TILE_OVERFLOW);
+  }
+}
+
+// One system or a batch: the block's particles, every copy placed.  Block 0 clears the word of the largest cell that
+// k_cell_scan finds.
+template <class T, int N, int SH, bool BATCH>
+__global__ void __launch_bounds__(WE_BLOCK) k_wrap_place(const __grid_constant__ PlaceArgs<T> P, int* __restrict__ max_cell) {
+  __shared__ PlaceShared<T, N, WE_BLOCK> sm;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *max_cell = 0;
+  if (!BATCH) load_shift<T>(P.g, sm.shift);
+  place_copies<T, N, SH, WE_BLOCK, BATCH>(P, blockIdx.x * WE_BLOCK, 32, sm);
+}
+
+// The gather after k_wrap_place and k_cell_scan.  A block takes `per` cells, which are a contiguous range of the cell
+// list: it reads their buckets into shared memory, ranks every copy by value within its cell (particle-index order,
+// rank_in_cell), and then walks the range in its final order, so that only the wrapped positions are read out of
+// order.  The scan words (`zero`, `zwords` 64-bit words) are cleared for the next build.
+constexpr int kGatherMax = 4096;   // values per block: per * slots
+constexpr int kGatherCells = 256;  // cells per block (8-bit cell numbers)
+template <class T, int N, bool BATCH>
+__global__ void __launch_bounds__(kBlock) k_bucket_gather(const __grid_constant__ PlaceArgs<T> P, const int* __restrict__ cell_sys,
+                                                          const int* __restrict__ cell_start, int ncells, int per, int cap,
+                                                          T* __restrict__ px, T* __restrict__ py, T* __restrict__ pz,
+                                                          float4* __restrict__ off, float4* __restrict__ xq,
+                                                          int* __restrict__ code, unsigned long long* __restrict__ zero,
+                                                          int64_t zwords) {
+  extern __shared__ uint32_t gather_smem[];
+  __shared__ T s_shift[27][3];
+  __shared__ int s_start[kGatherCells + 1];
+  uint32_t* vals = gather_smem;
+  uint32_t* sorted = vals + per * P.slots;
+  uint8_t* cell = reinterpret_cast<uint8_t*>(sorted + per * P.slots);
+  for (int64_t w = (int64_t)blockIdx.x * kBlock + threadIdx.x; w < zwords; w += (int64_t)gridDim.x * kBlock) zero[w] = 0ull;
+  const int c0 = blockIdx.x * per, nc = min(per, ncells - c0);
+  for (int t = threadIdx.x; t <= nc; t += kBlock) s_start[t] = cell_start[c0 + t];
+  if (!BATCH) load_shift<T>(P.g, s_shift);
+  if (*(volatile int*)P.err & DERR_TILE_OVERFLOW) return;  // set by k_wrap_place: the list is not used
+  __syncthreads();
+  const int base = s_start[0], tot = s_start[nc] - base;
+  if (tot < 0 || tot > per * P.slots || base < 0) {  // the same in every thread
+    if (threadIdx.x == 0) atomicOr(P.err, DERR_COPY_OVERFLOW);
+    return;
+  }
+  for (int e = threadIdx.x; e < tot; e += kBlock) {
+    int lo = 0, hi = nc;  // the last cell that starts at or before copy e
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (s_start[mid] - base <= e) lo = mid;
+      else hi = mid;
+    }
+    cell[e] = (uint8_t)lo;
+    const int slot = e - (s_start[lo] - base);
+    vals[e] = P.bucket[(int64_t)(c0 + lo) * P.slots + min(slot, P.slots - 1)];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < tot; e += kBlock) {
+    const int c = cell[e], s = s_start[c] - base, t = s_start[c + 1] - base;
+    const uint32_t v = vals[e];
+    const int r = s + rank_in_cell(vals, s, t, v);
+    if (r < t) sorted[r] = v;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < tot; e += kBlock) {
+    const uint32_t v = sorted[e];
+    const int p = (int)(v >> 5), k = (int)(v & 31u), t = base + e;
+    int li = c0 + cell[e];
+    if (t >= cap) {
+      atomicOr(P.err, DERR_COPY_OVERFLOW);
+      continue;
+    }
+    if (p >= P.n) {
+      atomicOr(P.err, DERR_CELL_RANGE);
+      continue;
+    }
+    T w[N];
+#pragma unroll
+    for (int d = 0; d < N; d++) w[d] = P.wrapped[(int64_t)p * N + d];
+    if constexpr (BATCH) {
+      const int s = cell_sys[li];
+      const DevGeom<T>& g = P.gtab[s];
+      li -= P.cbase[s];
+      if (k >= g.nimg || li < 0 || li >= g.ncells) {
+        atomicOr(P.err, DERR_CELL_RANGE);
+        continue;
+      }
+      gather_copy<T, N>(g, g.shift, w, t, p, k, li, px, py, pz, off, xq, code);
+    } else {
+      if (k >= P.g.nimg) {
+        atomicOr(P.err, DERR_CELL_RANGE);
+        continue;
+      }
+      gather_copy<T, N>(P.g, s_shift, w, t, p, k, li, px, py, pz, off, xq, code);
+    }
+  }
+}
+
 // ------------------------------------------------------------------ one system of few particles: one launch
 // The whole build in one cooperative kernel, for sets of at most kSmallParticles: the four kernels of the
 // counting build are each a few us of latency at these sizes.  Every warp wraps its particles (warps of
@@ -635,13 +830,9 @@ constexpr int64_t kSmallCells = 1 << 15;
 constexpr double kSmallPerCell = 64.0;  // copies per cell expected at uniform density: half a bucket
 
 template <class T> struct SmallBuild {
-  DevGeom<T> g;
-  const T* x;
-  int n, ncells, cap;
-  T* wrapped;
-  uint32_t* bucket;   // kBucket values per cell
-  int* cf;            // {copies, holds a real particle} per cell, zero on entry
-  int* cf_next;       // the next build's, cleared here
+  PlaceArgs<T> P;
+  int ncells, cap;
+  int* cf_next;       // the next build's counters, cleared here
   unsigned* bar;      // {arrived, generation}
   unsigned epoch;     // this launch's generation
   int* cell_start;
@@ -655,37 +846,19 @@ template <class T> struct SmallBuild {
   float4* off;
   float4* xq;
   int* code;
-  int* err;
 };
 
 template <class T, int N, int SH>
 __global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_constant__ SmallBuild<T> B) {
-  const DevGeom<T>& g = B.g;
+  const DevGeom<T>& g = B.P.g;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int kW = kSmallThreads / 32;
+  __shared__ PlaceShared<T, N, kSmallThreads> sm;
+  load_shift<T>(g, sm.shift);
   for (int c = blockIdx.x * kSmallThreads + threadIdx.x; c < 2 * B.ncells; c += gridDim.x * kSmallThreads) B.cf_next[c] = 0;
-  for (int i0 = (warp * gridDim.x + blockIdx.x) * 32; i0 < B.n; i0 += kW * gridDim.x * 32) {
-    const int i = i0 + lane;
-    if (i < B.n) {
-      T p[N];
-      uint32_t m = 0u;
-      int nc = 0;
-      if (!wrap_count_regs<T, N, SH>(g, B.x, i, p, m, nc)) atomicOr(B.err, DERR_NAN);
-#pragma unroll
-      for (int d = 0; d < N; d++) B.wrapped[(int64_t)i * N + d] = p[d];
-      for (int c = 0; c < nc; c++) {
-        int k = g.zero_code;
-        if (c > 0) {
-          k = lowest_bit(m);
-          m &= m - 1u;
-        }
-        const int key = copy_cell<T, N>(g, p, k, B.err);
-        const int slot = atomicAdd(&B.cf[2 * key], 1);
-        if (c == 0) B.cf[2 * key + 1] = 1;
-        if (slot < kBucket) B.bucket[(int64_t)key * kBucket + slot] = ((uint32_t)i << 5) | (uint32_t)k;
-        else atomicOr(B.err, DERR_TILE_OVERFLOW);
-      }
-    }
+  for (int i0 = blockIdx.x * 32; i0 < B.P.n; i0 += kW * gridDim.x * 32) {
+    place_copies<T, N, SH, kSmallThreads, false>(B.P, i0, (int)gridDim.x * 32, sm);
+    __syncthreads();
   }
   // ---- barrier over the grid (all blocks are resident: cooperative launch).  The last block to arrive opens it.
   __shared__ int s_ok;
@@ -701,7 +874,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_cons
       int spins = 0;
       while (*(volatile unsigned*)&B.bar[1] != B.epoch) {
         if (++spins > kScanSpinLimit) {
-          atomicOr(B.err, DERR_SCAN);
+          atomicOr(B.P.err, DERR_SCAN);
           s_ok = 0;
           break;
         }
@@ -718,7 +891,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_cons
   __shared__ int s_sum[2][kW];
   __shared__ int s_base[2];
   __shared__ int wsum_c[kW + 1], wsum_f[kW + 1];
-  const int2* cf2 = reinterpret_cast<const int2*>(B.cf);
+  const int2* cf2 = reinterpret_cast<const int2*>(B.P.cf);
   {
     int sc = 0, sf = 0;
     for (int c = threadIdx.x; c < c0; c += kSmallThreads) {
@@ -740,7 +913,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_cons
     }
     __syncthreads();
   }
-  const bool skip = (__ldcg(B.err) & (DERR_TILE_OVERFLOW | DERR_NAN)) != 0;  // the cell list is not used
+  const bool skip = (__ldcg(B.P.err) & (DERR_TILE_OVERFLOW | DERR_NAN)) != 0;  // the cell list is not used
   for (int cb = c0; cb < c1; cb += kSmallThreads) {  // 512 cells at a time
     const int c = cb + threadIdx.x;
     int2 v = make_int2(0, 0);
@@ -758,7 +931,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_cons
         *B.n_real = fpos + v.y;
         *B.max_cell = 0;
       }
-      if (start + v.x > B.cap) atomicOr(B.err, DERR_COPY_OVERFLOW);
+      if (start + v.x > B.cap) atomicOr(B.P.err, DERR_COPY_OVERFLOW);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -771,13 +944,13 @@ __global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_cons
   __syncthreads();  // the starts written above are read below by the block that wrote them
   for (int c = c0 + warp; c < c1; c += kW) {
     const int s = B.cell_start[c];
-    const int cnt = __ldcg(&B.cf[2 * c]);
+    const int cnt = __ldcg(&B.P.cf[2 * c]);
     if (cnt == 0 || s + cnt > B.cap) continue;
     uint32_t v[kBucket / 32];
     int r[kBucket / 32];
 #pragma unroll
     for (int q = 0; q < kBucket / 32; q++) {
-      v[q] = (32 * q + lane < cnt) ? __ldcg(&B.bucket[(int64_t)c * kBucket + 32 * q + lane]) : 0xffffffffu;
+      v[q] = (32 * q + lane < cnt) ? __ldcg(&B.P.bucket[(int64_t)c * kBucket + 32 * q + lane]) : 0xffffffffu;
       r[q] = 0;
     }
 #pragma unroll
@@ -793,14 +966,14 @@ __global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_cons
     for (int q = 0; q < kBucket / 32; q++) {
       if (32 * q + lane < cnt) {
         const int p = (int)(v[q] >> 5), k = (int)(v[q] & 31u);
-        if (p >= B.n || k >= g.nimg || r[q] >= cnt) {
-          atomicOr(B.err, DERR_CELL_RANGE);
+        if (p >= B.P.n || k >= g.nimg || r[q] >= cnt) {
+          atomicOr(B.P.err, DERR_CELL_RANGE);
           continue;
         }
         T w[N];
 #pragma unroll
-        for (int d = 0; d < N; d++) w[d] = __ldcg(&B.wrapped[(int64_t)p * N + d]);
-        gather_copy<T, N>(g, w, s + r[q], p, k, c, B.px, B.py, B.pz, B.off, B.xq, B.code);
+        for (int d = 0; d < N; d++) w[d] = __ldcg(&B.P.wrapped[(int64_t)p * N + d]);
+        gather_copy<T, N>(g, sm.shift, w, s + r[q], p, k, c, B.px, B.py, B.pz, B.off, B.xq, B.code);
       }
     }
   }
@@ -1081,14 +1254,17 @@ int build_small(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, i
   }
   S.small_epoch++;
   SmallBuild<T> B;
-  B.g = dg;
-  B.x = S.x.as<T>();
-  B.n = (int)n;
+  std::memset((void*)&B, 0, sizeof B);
+  B.P.g = dg;
+  B.P.x = S.x.as<T>();
+  B.P.n = (int)n;
+  B.P.wrapped = S.wrapped.as<T>();
+  B.P.bucket = S.small_buf.as<uint32_t>() + words;
+  B.P.slots = kBucket;
+  B.P.cf = S.small_buf.as<int>() + ((S.small_epoch & 1) ? 2 * ncells : 0);
+  B.P.err = h.err.as<int>();
   B.ncells = (int)ncells;
   B.cap = (int)cap;
-  B.wrapped = S.wrapped.as<T>();
-  B.bucket = S.small_buf.as<uint32_t>() + words;
-  B.cf = S.small_buf.as<int>() + ((S.small_epoch & 1) ? 2 * ncells : 0);
   B.cf_next = S.small_buf.as<int>() + ((S.small_epoch & 1) ? 0 : 2 * ncells);
   B.bar = reinterpret_cast<unsigned*>(S.small_buf.as<int>() + 4 * ncells);
   B.epoch = S.small_epoch;
@@ -1103,7 +1279,6 @@ int build_small(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, i
   B.off = S.off.as<float4>();
   B.xq = S.xq.as<float4>();
   B.code = S.code.as<int>();
-  B.err = h.err.as<int>();
   void* args[] = {&B};
   const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k, dim3((unsigned)sms), dim3(kSmallThreads), args, 0, h.stream);
   if (e != cudaSuccess) S.small_cells = 0;
@@ -1180,8 +1355,8 @@ int build_counting(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n
   CLM_CUDA_TRY(h, cudaGetLastError());
   h.launches++;
   k_cell_scan<<<(unsigned)ct, kBlock, 0, h.stream>>>(cell_cf, (int)ncells, S.cell_start.as<int>(), S.cell_flags.as<int>(),
-                                                     S.real_list.as<int>(), S.real_scan.as<int>() + ncells, max_cell,
-                                                     st_c, st_f, reinterpret_cast<unsigned*>(st_c + ct), (int)ct, err);
+                                                     S.real_list.as<int>(), nullptr, S.real_scan.as<int>() + ncells,
+                                                     max_cell, st_c, st_f, reinterpret_cast<unsigned*>(st_c + ct), (int)ct, err);
   CLM_CUDA_TRY(h, cudaGetLastError());
   h.launches++;
   k_cell_scatter<<<(unsigned)tiles, kBlock, 0, h.stream>>>(S.keys[0].as<uint32_t>(), S.vals[0].as<uint32_t>(),
@@ -1204,6 +1379,92 @@ int build_counting(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n
                                                      (int)cap, (int)n, S.px.as<T>(), S.py.as<T>(), S.pz.as<T>(),
                                                      S.off.as<float4>(), S.xq.as<float4>(), S.code.as<int>(),
                                                      S.cell_flags.as<int>(), z, zwords, err);
+  CLM_CUDA_TRY(h, cudaGetLastError());
+  h.launches++;
+  S.cell_count_zero = zero_bytes;
+  return OK;
+}
+
+// Places per cell of k_wrap_place's buckets (0: the set is not for them).  `e` is the number of copies expected in a
+// cell, `densest` the same in the densest system of a batch: seven standard deviations of a Poisson count above it, so
+// that uniform sets never overflow.  Cells of more than 64 copies (their ranks cost a cell's size per copy) and grids
+// of mostly empty cells (the buckets would take more memory than the copies) go to the other builds.
+constexpr int kBucketMost = 256;
+template <class T> int bucket_slots(const SetData& S, double e, double densest, int64_t ncells, int64_t cap) {
+  if (S.bucket_off || S.prefer_radix || !(e <= kCountingMaxPerCell) || !(densest < (double)kBucketMost)) return 0;
+  const int slots = std::max(S.bucket, ((int)(densest + 7.0 * std::sqrt(densest) + 8.0) + 7) / 8 * 8);
+  return slots <= kBucketMost && (double)ncells * slots <= 16.0 * (double)cap + 65536.0 ? slots : 0;
+}
+
+// One system, or a batch (one cell list over the global cell index): wrap, images and placement (k_wrap_place), cell
+// starts and real cells (k_cell_scan), ranks and gather (k_bucket_gather).
+template <class T>
+int build_bucket(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, int64_t ncells, int64_t cap, int slots) {
+  const bool batch = h.batch.on;
+  int* err = h.err.as<int>();
+  const int64_t ct = (ncells + SCAN_TILE - 1) / SCAN_TILE;
+  // the same region as the counting build's: scan words of the copies and their ticket, of the flags, then the counters
+  const int64_t w_c = ct + 1, w_f = ct;
+  const size_t zero_bytes = sizeof(unsigned long long) * (size_t)(w_c + w_f + ncells + 1);
+  const void* zero_at = S.cell_count.p;
+  if (!S.cell_count.reserve(zero_bytes) || !S.wrapped.reserve(sizeof(T) * N * n) ||
+      !S.keys[0].reserve(sizeof(uint32_t) * (size_t)ncells * slots) || !S.px.reserve(sizeof(T) * cap) ||
+      !S.py.reserve(sizeof(T) * cap) || !S.pz.reserve(sizeof(T) * cap) ||
+      !S.off.reserve(std::is_same<T, float>::value ? 16 : sizeof(float4) * cap) || !S.code.reserve(sizeof(int) * cap) ||
+      !S.xq.reserve(std::is_same<T, float>::value ? sizeof(float4) * cap : 16))
+    return ERR_NOMEM;
+  if (S.cell_count.p != zero_at) S.cell_count_zero = 0;  // a new allocation holds no cleared words
+  unsigned long long* st_c = S.cell_count.as<unsigned long long>();
+  unsigned long long* st_f = st_c + w_c;
+  int* cell_cf = reinterpret_cast<int*>(st_f + w_f);
+  // cleared by the previous build unless the region grew or moved
+  if (S.cell_count_zero < zero_bytes) CLM_CUDA_TRY(h, cudaMemsetAsync(st_c, 0, zero_bytes, h.stream));
+  S.cell_count_zero = 0;
+  int* max_cell = S.copy_off.as<int>() + n + 1;  // the largest cell
+  PlaceArgs<T> P;
+  std::memset((void*)&P, 0, sizeof P);
+  P.g = dg;
+  P.gtab = h.batch.gtab.as<DevGeom<T>>();
+  P.psys = h.batch.psys.as<int>();
+  P.cbase = h.batch.cbase_d.as<int>();
+  P.sys_err = h.batch.sys_err.as<int>();
+  P.x = S.x.as<T>();
+  P.n = (int)n;
+  P.wrapped = S.wrapped.as<T>();
+  P.bucket = S.keys[0].as<uint32_t>();
+  P.slots = slots;
+  P.cf = cell_cf;
+  P.err = err;
+  using Place = void (*)(const PlaceArgs<T>, int*);
+  Place place;
+  if (batch) place = (N == 3) ? (Place)k_wrap_place<T, 3, kShapeGeneral, true> : (Place)k_wrap_place<T, 2, kShapeGeneral, true>;
+  else place = (N == 3) ? (Place)k_wrap_place<T, 3, kShapeGeneral, false> : (Place)k_wrap_place<T, 2, kShapeGeneral, false>;
+  if constexpr (std::is_same<T, double>::value) {
+    // Float64 3D cells whose input matrix has exact zeros take a wrap that skips them (wrap_point_shaped)
+    if (!batch && N == 3 && dg.shape == kShapeDiag) place = k_wrap_place<T, 3, kShapeDiag, false>;
+    else if (!batch && N == 3 && dg.shape == kShapeUpper) place = k_wrap_place<T, 3, kShapeUpper, false>;
+  }
+  place<<<(unsigned)((n + WE_BLOCK - 1) / WE_BLOCK), WE_BLOCK, 0, h.stream>>>(P, max_cell);
+  CLM_CUDA_TRY(h, cudaGetLastError());
+  h.launches++;
+  k_cell_scan<<<(unsigned)ct, kBlock, 0, h.stream>>>(cell_cf, (int)ncells, S.cell_start.as<int>(), S.cell_flags.as<int>(),
+                                                     S.real_list.as<int>(), batch ? S.real_scan.as<int>() : nullptr,
+                                                     S.real_scan.as<int>() + ncells, max_cell, st_c, st_f,
+                                                     reinterpret_cast<unsigned*>(st_c + ct), (int)ct, err);
+  CLM_CUDA_TRY(h, cudaGetLastError());
+  h.launches++;
+  // about 512 copies per block
+  const int most = std::min(kGatherMax / slots, kGatherCells);
+  const int per = (int)std::max(1.0, std::min((double)most, 512.0 * (double)ncells / (double)cap));
+  const size_t smem = (size_t)per * slots * 9;
+  using Gather = void (*)(const PlaceArgs<T>, const int*, const int*, int, int, int, T*, T*, T*, float4*, float4*, int*,
+                          unsigned long long*, int64_t);
+  Gather gather;
+  if (batch) gather = (N == 3) ? (Gather)k_bucket_gather<T, 3, true> : (Gather)k_bucket_gather<T, 2, true>;
+  else gather = (N == 3) ? (Gather)k_bucket_gather<T, 3, false> : (Gather)k_bucket_gather<T, 2, false>;
+  gather<<<(unsigned)((ncells + per - 1) / per), kBlock, smem, h.stream>>>(
+      P, h.batch.cell_sys.as<int>(), S.cell_start.as<int>(), (int)ncells, per, (int)cap, S.px.as<T>(), S.py.as<T>(),
+      S.pz.as<T>(), S.off.as<float4>(), S.xq.as<float4>(), S.code.as<int>(), st_c, w_c + w_f);
   CLM_CUDA_TRY(h, cudaGetLastError());
   h.launches++;
   S.cell_count_zero = zero_bytes;
@@ -1267,11 +1528,23 @@ template <class T> int build_set(Handle& h, int set, const Geometry<T>& g) {
   const bool crowded = !batch && (S.prefer_radix || (double)cap > kCountingMaxPerCell * (double)ncells);
   S.counted = !batch && !crowded;
   S.small = false;
+  S.bucket_used = 0;
   if (!batch && !S.prefer_radix && !S.small_off && n <= kSmallParticles && ncells <= kSmallCells &&
       copies_expected(S, g) <= kSmallPerCell * (double)ncells) {
     const int st = build_small<T>(h, S, dg, N, n, ncells, cap, &S.small);
     if (S.small) S.counted = true;
     if (st || S.small) return st;
+  }
+  double per_cell = (double)n;  // copies per cell at uniform density
+  if (!batch)
+    for (int i = 0; i < N; i++)  // without a periodic cell the particles fill the grid but for its margins
+      per_cell *= g.kind == NONPERIODIC ? 1.0 / std::max(1.0, (double)(g.nc[i] - 2 * g.lcell - 1)) : (double)g.cs[i];
+  if (!batch && g.kind != NONPERIODIC) per_cell /= std::fabs((double)g.det_in);
+  if (batch && ncells > 0) S.bucket_used = bucket_slots<T>(S, h.batch.copies_est / (double)ncells, h.batch.cell_est, ncells, cap);
+  else if (!batch) S.bucket_used = bucket_slots<T>(S, per_cell, per_cell, ncells, cap);
+  if (S.bucket_used) {
+    S.counted = true;
+    return build_bucket<T>(h, S, dg, N, n, ncells, cap, S.bucket_used);
   }
   if (S.counted) return build_counting<T>(h, S, dg, N, n, ncells, cap);
   // the radix path's gather sets the real flags of the cells it fills
@@ -1462,7 +1735,16 @@ int check_build_totals(Handle& h, bool* overflow) {
     if (S.counted && h.pinned[44 + s] > kRadixAbovePerCell) S.prefer_radix = true;
     if (S.small && (errw & DERR_TILE_OVERFLOW)) {
       // a cell had more copies than its bucket: the counting build (or radix, when it finds the cell crowded)
-      S.small_off = true;
+      S.small_off = S.bucket_off = true;
+      S.dirty = true;
+      *overflow = true;
+    } else if (S.bucket_used && (errw & DERR_TILE_OVERFLOW)) {
+      // more places than the largest cell's copies, or the other builds
+      const int most = h.pinned[44 + s], want = (most + most / 4 + 7) / 8 * 8;
+      if (most > S.bucket_used) {
+        if (want <= kBucketMost) S.bucket = want;
+        else S.bucket_off = true;
+      }
       S.dirty = true;
       *overflow = true;
     } else if (S.counted && (errw & DERR_TILE_OVERFLOW)) {

@@ -293,21 +293,23 @@ __host__ __device__ __forceinline__ bool wrap_count_at(const DevGeom<T>& g, cons
 // The cell of image k of a particle at wrapped position p (k = zero_code: the real copy, with the border-case
 // shift); an out-of-range cell is flagged and mapped to cell 0.
 template <class T, int N>
-__host__ __device__ __forceinline__ int copy_cell(const DevGeom<T>& g, const T* p, int k, int* __restrict__ err) {
-  int li;
-  if (k == g.zero_code) {
-    li = cell_of<T, N>(g, p, true);
-  } else {
-    T q[N];
+__host__ __device__ __forceinline__ int copy_cell(const DevGeom<T>& g, const T (*shift)[3], const T* p, int k,
+                                                  int* __restrict__ err) {
+  // `shift` is g.shift, or a copy of it in shared memory (lanes read different rows, which the constant bank
+  // serves one after the other)
+  T q[N];
 #pragma unroll
-    for (int d = 0; d < N; d++) q[d] = xadd(p[d], g.shift[k][d]);
-    li = cell_of<T, N>(g, q, false);
-  }
+  for (int d = 0; d < N; d++) q[d] = (k == g.zero_code) ? p[d] : xadd(p[d], shift[k][d]);
+  int li = cell_of<T, N>(g, q, k == g.zero_code);
   if (li < 0) {
     flag_error(err, DERR_CELL_RANGE);
     li = 0;
   }
   return li;
+}
+template <class T, int N>
+__host__ __device__ __forceinline__ int copy_cell(const DevGeom<T>& g, const T* p, int k, int* __restrict__ err) {
+  return copy_cell<T, N>(g, g.shift, p, k, err);
 }
 
 // The copies of particle i (wrapped position p, image mask m, ncp copies) at copy positions base .. base+ncp-1:
@@ -436,14 +438,15 @@ __host__ __device__ __forceinline__ void cell_starts_at(const uint32_t* __restri
 }
 
 // Copy t of the cell list: image k of particle p, at wrapped position w, in the cell `li` (local index of its
-// system).
+// system); `shift` as in copy_cell.
 template <class T, int N>
-__host__ __device__ __forceinline__ void gather_copy(const DevGeom<T>& g, const T* w, int t, int p, int k, int li,
+__host__ __device__ __forceinline__ void gather_copy(const DevGeom<T>& g, const T (*shift)[3], const T* w, int t, int p, int k,
+                                            int li,
                                             T* __restrict__ px, T* __restrict__ py, T* __restrict__ pz,
                                             float4* __restrict__ off, float4* __restrict__ xq, int* __restrict__ code) {
   T q[N];
 #pragma unroll
-  for (int d = 0; d < N; d++) q[d] = (k == g.zero_code) ? w[d] : xadd(w[d], g.shift[k][d]);
+  for (int d = 0; d < N; d++) q[d] = (k == g.zero_code) ? w[d] : xadd(w[d], shift[k][d]);
   const int pc = (k == g.zero_code) ? p : -(p + 1);
   px[t] = q[0];
   py[t] = q[1];
@@ -476,7 +479,7 @@ __host__ __device__ __forceinline__ void gather_at(const DevGeom<T>& g, const T*
   T w[N];
 #pragma unroll
   for (int d = 0; d < N; d++) w[d] = wrapped[(int64_t)p * N + d];
-  gather_copy<T, N>(g, w, t, p, k, li, px, py, pz, off, xq, code);
+  gather_copy<T, N>(g, g.shift, w, t, p, k, li, px, py, pz, off, xq, code);
   if (k == g.zero_code) cell_flags[cb + li] = 1;  // the cell holds a real particle
 }
 

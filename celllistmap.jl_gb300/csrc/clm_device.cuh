@@ -183,6 +183,33 @@ template <class T> __host__ __device__ __forceinline__ bool is_zero_bits(T v) { 
 template <class T> __host__ __device__ __forceinline__ bool is_finite_bits(T v) {
   return mag_bits(v) < (sizeof(T) == 8 ? 0x7FF0000000000000ull : 0x7F800000ull);
 }
+#ifdef __CUDA_ARCH__
+// On the two words: the compiler turns the 64-bit forms back into FP64 compares.
+__device__ __forceinline__ bool is_zero_bits(double v) {
+  return (((unsigned)__double2hiint(v) << 1) | (unsigned)__double2loint(v)) == 0u;
+}
+__device__ __forceinline__ bool is_finite_bits(double v) { return ((unsigned)__double2hiint(v) << 1) < 0xFFE00000u; }
+#endif
+// 0 < v < 1
+__host__ __device__ __forceinline__ bool inside_unit(double v) {
+  return (unsigned long long)dbits(v) - 1ull < 0x3FF0000000000000ull - 1ull;
+}
+__host__ __device__ __forceinline__ bool inside_unit(float v) {
+#ifdef __CUDA_ARCH__
+  const unsigned b = __float_as_uint(v);
+#else
+  unsigned b;
+  std::memcpy(&b, &v, sizeof b);
+#endif
+  return b - 1u < 0x3F800000u - 1u;
+}
+// Fraction of a cell coordinate: fastmod1, with the boundary (1) at 0.  A coordinate inside the unit cell is its own
+// fraction (its floor is +0), so a particle that is there already takes no FP64 step.
+template <class T> __host__ __device__ __forceinline__ T unit_fraction(T v) {
+  if (inside_unit(v)) return v;
+  const T f = xsub(v, xfloor(v));
+  return same_bits(f, T(1)) ? T(0) : f;  // f == 1 (the only value equal to 1 is 1), on the integer pipe
+}
 
 // Cell shapes whose wrap skips exact-zero terms (DevGeom::shape; 3D only).  A left-to-right sum of separately
 // rounded products whose dropped terms are signed zeros (a zero coefficient times a finite value) equals the
@@ -210,9 +237,7 @@ __host__ __device__ __forceinline__ bool wrap_point_shaped(const DevGeom<T>& g, 
   if (is_zero_bits(p[0]) || is_zero_bits(p[1]) || is_zero_bits(p[2])) return false;
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    p[i] = quot_rn(p[i], g.det_in, g.inv_det);
-    p[i] = xsub(p[i], xfloor(p[i]));
-    if (same_bits(p[i], T(1))) p[i] = T(0);
+    p[i] = unit_fraction(quot_rn(p[i], g.det_in, g.inv_det));
   }
   T w[3];
   if constexpr (SH == kShapeDiag) {
@@ -256,10 +281,7 @@ __host__ __device__ __forceinline__ void wrap_point(const DevGeom<T>& g, const T
     p[1] = xdiv(xsub(xmul(a[0][0], x[1]), xmul(a[1][0], x[0])), g.det_in);
   }
 #pragma unroll
-  for (int i = 0; i < N; i++) {
-    p[i] = xsub(p[i], xfloor(p[i]));
-    if (same_bits(p[i], T(1))) p[i] = T(0);  // p == 1 (the only value equal to 1 is 1), on the integer pipe
-  }
+  for (int i = 0; i < N; i++) p[i] = unit_fraction(p[i]);
   T w[N];
 #pragma unroll
   for (int i = 0; i < N; i++) {

@@ -95,6 +95,10 @@ struct SetData {
   unsigned small_epoch = 0;  // launches since then
   bool small = false;        // the last build was one
   bool small_off = false;    // one met a cell with more copies than a bucket holds
+  // larger sets and batches: a bucket per cell (k_wrap_place)
+  int bucket_used = 0;       // places per cell of the last build (0: another build)
+  int bucket = 0;            // places that an earlier build's largest cell called for
+  bool bucket_off = false;   // one met a cell with more copies than a bucket may hold
 };
 
 struct ScanTemp {
@@ -116,6 +120,7 @@ struct BatchState {
   int64_t ncells = 0;            // total cells
   double real_cells = 0;         // cells with real particles (geometric estimate)
   double copies_est = 0;         // reals + images (uniform-density estimate)
+  double cell_est = 0;           // copies per cell of the densest system (likewise)
   double pairs_est = 0;          // pairs within the cutoff (uniform-density estimate)
   bool tables_ready = false;     // device tables match (systems, lcell, precision)
   int tables_dtype = -1;
