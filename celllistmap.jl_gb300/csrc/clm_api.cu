@@ -95,12 +95,12 @@ template <class T> int build_all(Handle& h, bool sync) {
         geom<T>(h) = g;
       }
     }
-    for (int s = 0; s < h.nsets; s++) {
-      SetData& S = h.sets[s];
-      if (S.dirty || !S.built || rebuild_all) {
-        int st = build_set<T>(h, s, geom<T>(h));
-        if (st) return st;
-      }
+    unsigned which = 0;
+    for (int s = 0; s < h.nsets; s++)
+      if (h.sets[s].dirty || !h.sets[s].built || rebuild_all) which |= 1u << s;
+    {
+      const int st = build_sets<T>(h, geom<T>(h), which);
+      if (st) return st;
     }
     cudaEventRecord(h.ev[1], h.stream);
     if (!sync) {

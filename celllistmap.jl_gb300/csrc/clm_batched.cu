@@ -346,7 +346,7 @@ template <class T> int enqueue_op(Handle& h, int slot, int op, const clm_op_para
 template <class T> int enqueue_step(Handle& h, int nops, const int* ops, const clm_op_params* P) {
   BatchState& B = h.batch;
   CLM_CUDA_TRY(h, cudaMemsetAsync(h.err.p, 0, 64, h.stream));
-  int st = build_set<T>(h, 0, tmpl_geom<T>(h));
+  int st = build_sets<T>(h, tmpl_geom<T>(h), 1u);
   if (st) return st;
   for (int k = 0; k < nops; k++) {
     st = enqueue_op<T>(h, k, ops[k], P ? &P[k] : nullptr);

@@ -626,7 +626,6 @@ __global__ void __launch_bounds__(kBlock) k_rank_gather(DevGeom<T> g, const T* _
 // copy, a few have seven, and lanes that walked their own would leave the others idle (and in Float64 hold the FP64
 // pipe, 16 cycles per warp instruction, for each round).
 template <class T> struct PlaceArgs {
-  DevGeom<T> g;
   const DevGeom<T>* gtab;  // batches: geometry per system, system of each particle, first cell of each system
   const int* psys;
   const int* cbase;
@@ -652,7 +651,8 @@ template <class T> __device__ __forceinline__ void load_shift(const DevGeom<T>& 
 // Particles first + warp * stride + lane of one block of NT threads (at most 2048).  One system: sm.shift holds the
 // geometry's shifts (visible after the scan's barriers).
 template <class T, int N, int SH, int NT, bool BATCH>
-__device__ __forceinline__ void place_copies(const PlaceArgs<T>& P, int first, int stride, PlaceShared<T, N, NT>& sm) {
+__device__ __forceinline__ void place_copies(const DevGeom<T>& G, const PlaceArgs<T>& P, int first, int stride,
+                                             PlaceShared<T, N, NT>& sm) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i = first + warp * stride + lane;
   T p[N];
@@ -672,7 +672,7 @@ __device__ __forceinline__ void place_copies(const PlaceArgs<T>& P, int first, i
         if (!ok) atomicOr(&P.sys_err[s], DERR_NAN);
       }
     } else {
-      ok = wrap_count_regs<T, N, SH>(P.g, P.x, i, p, m, v[0]);
+      ok = wrap_count_regs<T, N, SH>(G, P.x, i, p, m, v[0]);
       if (!ok) atomicOr(P.err, DERR_NAN);
     }
 #pragma unroll
@@ -685,7 +685,7 @@ __device__ __forceinline__ void place_copies(const PlaceArgs<T>& P, int first, i
   int off = 0;
   const int agg = block_scan<1, NT>(v, off, sm.wsum);
   if (nc > 0) {
-    const int zero = BATCH ? (N == 3 ? 13 : 4) : P.g.zero_code;
+    const int zero = BATCH ? (N == 3 ? 13 : 4) : G.zero_code;
     uint16_t* at = sm.list + off + v[0];
     *at++ = (uint16_t)(threadIdx.x << 5 | zero);
     while (m) {
@@ -706,8 +706,8 @@ __device__ __forceinline__ void place_copies(const PlaceArgs<T>& P, int first, i
       key = P.cbase[sm.sys[t]] + copy_cell<T, N>(g, q, k, P.err);
       real = k == (N == 3 ? 13 : 4);
     } else {
-      key = copy_cell<T, N>(P.g, sm.shift, q, k, P.err);
-      real = k == P.g.zero_code;
+      key = copy_cell<T, N>(G, sm.shift, q, k, P.err);
+      real = k == G.zero_code;
     }
     const int slot = atomicAdd(&P.cf[2 * (int64_t)key], 1);
     if (real) P.cf[2 * (int64_t)key + 1] = 1;
@@ -720,11 +720,12 @@ __device__ __forceinline__ void place_copies(const PlaceArgs<T>& P, int first, i
 // One system or a batch: the block's particles, every copy placed.  Block 0 clears the word of the largest cell that
 // k_cell_scan finds.
 template <class T, int N, int SH, bool BATCH>
-__global__ void __launch_bounds__(WE_BLOCK) k_wrap_place(const __grid_constant__ PlaceArgs<T> P, int* __restrict__ max_cell) {
+__global__ void __launch_bounds__(WE_BLOCK) k_wrap_place(const __grid_constant__ DevGeom<T> G,
+                                                         const __grid_constant__ PlaceArgs<T> P, int* __restrict__ max_cell) {
   __shared__ PlaceShared<T, N, WE_BLOCK> sm;
   if (blockIdx.x == 0 && threadIdx.x == 0) *max_cell = 0;
-  if (!BATCH) load_shift<T>(P.g, sm.shift);
-  place_copies<T, N, SH, WE_BLOCK, BATCH>(P, blockIdx.x * WE_BLOCK, 32, sm);
+  if (!BATCH) load_shift<T>(G, sm.shift);
+  place_copies<T, N, SH, WE_BLOCK, BATCH>(G, P, blockIdx.x * WE_BLOCK, 32, sm);
 }
 
 // The gather after k_wrap_place and k_cell_scan.  A block takes `per` cells, which are a contiguous range of the cell
@@ -734,8 +735,8 @@ __global__ void __launch_bounds__(WE_BLOCK) k_wrap_place(const __grid_constant__
 constexpr int kGatherMax = 4096;   // values per block: per * slots
 constexpr int kGatherCells = 256;  // cells per block (8-bit cell numbers)
 template <class T, int N, bool BATCH>
-__global__ void __launch_bounds__(kBlock) k_bucket_gather(const __grid_constant__ PlaceArgs<T> P, const int* __restrict__ cell_sys,
-                                                          const int* __restrict__ cell_start, int ncells, int per, int cap,
+__global__ void __launch_bounds__(kBlock) k_bucket_gather(const __grid_constant__ DevGeom<T> G, const __grid_constant__ PlaceArgs<T> P,
+                                                          const int* __restrict__ cell_sys, const int* __restrict__ cell_start, int ncells, int per, int cap,
                                                           T* __restrict__ px, T* __restrict__ py, T* __restrict__ pz,
                                                           float4* __restrict__ off, float4* __restrict__ xq,
                                                           int* __restrict__ code, unsigned long long* __restrict__ zero,
@@ -749,7 +750,7 @@ __global__ void __launch_bounds__(kBlock) k_bucket_gather(const __grid_constant_
   for (int64_t w = (int64_t)blockIdx.x * kBlock + threadIdx.x; w < zwords; w += (int64_t)gridDim.x * kBlock) zero[w] = 0ull;
   const int c0 = blockIdx.x * per, nc = min(per, ncells - c0);
   for (int t = threadIdx.x; t <= nc; t += kBlock) s_start[t] = cell_start[c0 + t];
-  if (!BATCH) load_shift<T>(P.g, s_shift);
+  if (!BATCH) load_shift<T>(G, s_shift);
   if (*(volatile int*)P.err & DERR_TILE_OVERFLOW) return;  // set by k_wrap_place: the list is not used
   __syncthreads();
   const int base = s_start[0], tot = s_start[nc] - base;
@@ -801,11 +802,11 @@ __global__ void __launch_bounds__(kBlock) k_bucket_gather(const __grid_constant_
       }
       gather_copy<T, N>(g, g.shift, w, t, p, k, li, px, py, pz, off, xq, code);
     } else {
-      if (k >= P.g.nimg) {
+      if (k >= G.nimg) {
         atomicOr(P.err, DERR_CELL_RANGE);
         continue;
       }
-      gather_copy<T, N>(P.g, s_shift, w, t, p, k, li, px, py, pz, off, xq, code);
+      gather_copy<T, N>(G, s_shift, w, t, p, k, li, px, py, pz, off, xq, code);
     }
   }
 }
@@ -829,7 +830,7 @@ constexpr int64_t kSmallParticles = 1 << 16;
 constexpr int64_t kSmallCells = 1 << 15;
 constexpr double kSmallPerCell = 64.0;  // copies per cell expected at uniform density: half a bucket
 
-template <class T> struct SmallBuild {
+template <class T> struct SmallSet {
   PlaceArgs<T> P;
   int ncells, cap;
   int* cf_next;       // the next build's counters, cleared here
@@ -848,25 +849,36 @@ template <class T> struct SmallBuild {
   int* code;
 };
 
+// Both sets of an x-y handle in one launch: blocks [0, split) build set 0, the others set 1, each group with its own
+// barrier.
+template <class T> struct SmallBuild {
+  DevGeom<T> g;
+  SmallSet<T> set[2];
+  int split;
+};
+
 template <class T, int N, int SH>
-__global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_constant__ SmallBuild<T> B) {
-  const DevGeom<T>& g = B.P.g;
+__global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_constant__ SmallBuild<T> A) {
+  const DevGeom<T>& g = A.g;
+  const bool second = (int)blockIdx.x >= A.split;
+  const SmallSet<T>& B = A.set[second ? 1 : 0];
+  const int block = (int)blockIdx.x - (second ? A.split : 0), blocks = second ? (int)gridDim.x - A.split : A.split;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int kW = kSmallThreads / 32;
   __shared__ PlaceShared<T, N, kSmallThreads> sm;
   load_shift<T>(g, sm.shift);
-  for (int c = blockIdx.x * kSmallThreads + threadIdx.x; c < 2 * B.ncells; c += gridDim.x * kSmallThreads) B.cf_next[c] = 0;
-  for (int i0 = blockIdx.x * 32; i0 < B.P.n; i0 += kW * gridDim.x * 32) {
-    place_copies<T, N, SH, kSmallThreads, false>(B.P, i0, (int)gridDim.x * 32, sm);
+  for (int c = block * kSmallThreads + threadIdx.x; c < 2 * B.ncells; c += blocks * kSmallThreads) B.cf_next[c] = 0;
+  for (int i0 = block * 32; i0 < B.P.n; i0 += kW * blocks * 32) {
+    place_copies<T, N, SH, kSmallThreads, false>(g, B.P, i0, blocks * 32, sm);
     __syncthreads();
   }
-  // ---- barrier over the grid (all blocks are resident: cooperative launch).  The last block to arrive opens it.
+  // ---- barrier over the set's blocks (all are resident: cooperative launch).  The last block to arrive opens it.
   __shared__ int s_ok;
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     s_ok = 1;
-    if (atomicAdd(&B.bar[0], 1u) == gridDim.x - 1) {
+    if (atomicAdd(&B.bar[0], 1u) == (unsigned)blocks - 1u) {
       B.bar[0] = 0u;
       __threadfence();
       atomicExch(&B.bar[1], B.epoch);
@@ -886,8 +898,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_cons
   __syncthreads();
   if (!s_ok) return;
   // ---- this block's cells; what other blocks wrote is read past L1 (__ldcg)
-  const int per = (B.ncells + gridDim.x - 1) / gridDim.x;
-  const int c0 = min(B.ncells, (int)blockIdx.x * per), c1 = min(B.ncells, c0 + per);
+  const int per = (B.ncells + blocks - 1) / blocks;
+  const int c0 = min(B.ncells, block * per), c1 = min(B.ncells, c0 + per);
   __shared__ int s_sum[2][kW];
   __shared__ int s_base[2];
   __shared__ int wsum_c[kW + 1], wsum_f[kW + 1];
@@ -1083,44 +1095,101 @@ __global__ void k_compact(const int* __restrict__ flags, const int* __restrict__
   if (flags[li]) list[scanned[li]] = li;
 }
 
-template <class T, int N>
-__global__ void __launch_bounds__(kBlock) k_minmax(const T* __restrict__ x, int n, T* __restrict__ part) {
-  __shared__ T smin[N][kBlock], smax[N][kBlock];
+// Limits of both sets in one launch: a block reduces its share of a set (blockIdx.y) to partials, and the last block
+// of each set to finish reduces those and writes {lo, hi} to the host's pinned words.  The host needs the limits
+// before it can lay out the cells, so this is latency only: one launch and one wait, not a launch, a copy through
+// pageable memory and a wait per set (with the one launch of k_build_small for both sets, the build of 1501 and 4507
+// points went from 82 to 42 us).
+constexpr int kLimitBlocks = 256;
+template <class T> struct LimitArgs {
+  const T* x[2];
+  int n[2];
+  T* part;            // kLimitBlocks x 2N per set
+  unsigned* ticket;   // one per set, zero; left zero
+  T* out;             // pinned: 6 per set
+};
+template <class T, int N> __global__ void __launch_bounds__(kBlock) k_limits(const __grid_constant__ LimitArgs<T> A) {
+  __shared__ T s_v[kBlock / 32][2 * N];
+  __shared__ bool s_last;
+  const int set = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n = A.n[set];
+  if (n <= 0) return;
+  const int blocks = min((int)gridDim.x, (n + kBlock - 1) / kBlock);
+  if ((int)blockIdx.x >= blocks) return;
   T lo[N], hi[N];
+  const auto reduce = [&]() {  // the block's limits, in lo and hi of warp 0
+#pragma unroll
+    for (int d = 0; d < N; d++) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+        hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+      }
+      if (lane == 0) {
+        s_v[warp][d] = lo[d];
+        s_v[warp][N + d] = hi[d];
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+      for (int d = 0; d < N; d++) {
+        lo[d] = s_v[lane % (kBlock / 32)][d];
+        hi[d] = s_v[lane % (kBlock / 32)][N + d];
+#pragma unroll
+        for (int o = kBlock / 64; o > 0; o >>= 1) {
+          lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+          hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+        }
+      }
+    }
+  };
 #pragma unroll
   for (int d = 0; d < N; d++) {
     lo[d] = INFINITY;
     hi[d] = -INFINITY;
   }
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (int i = blockIdx.x * kBlock + threadIdx.x; i < n; i += blocks * kBlock) {
 #pragma unroll
     for (int d = 0; d < N; d++) {
-      T v = x[(int64_t)i * N + d];
+      const T v = A.x[set][(int64_t)i * N + d];
       lo[d] = fmin(lo[d], v);
       hi[d] = fmax(hi[d], v);
     }
   }
-#pragma unroll
-  for (int d = 0; d < N; d++) {
-    smin[d][threadIdx.x] = lo[d];
-    smax[d][threadIdx.x] = hi[d];
-  }
-  __syncthreads();
-  for (int s = kBlock / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) {
-#pragma unroll
-      for (int d = 0; d < N; d++) {
-        smin[d][threadIdx.x] = fmin(smin[d][threadIdx.x], smin[d][threadIdx.x + s]);
-        smax[d][threadIdx.x] = fmax(smax[d][threadIdx.x], smax[d][threadIdx.x + s]);
-      }
-    }
-    __syncthreads();
-  }
+  reduce();
+  T* part = A.part + (int64_t)set * kLimitBlocks * 2 * N;
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int d = 0; d < N; d++) {
-      part[(int64_t)blockIdx.x * 2 * N + d] = smin[d][0];
-      part[(int64_t)blockIdx.x * 2 * N + N + d] = smax[d][0];
+      part[(int64_t)blockIdx.x * 2 * N + d] = lo[d];
+      part[(int64_t)blockIdx.x * 2 * N + N + d] = hi[d];
+    }
+    __threadfence();
+    s_last = atomicAdd(&A.ticket[set], 1u) == (unsigned)blocks - 1u;
+  }
+  __syncthreads();
+  if (!s_last) return;
+#pragma unroll
+  for (int d = 0; d < N; d++) {
+    lo[d] = INFINITY;
+    hi[d] = -INFINITY;
+  }
+  __threadfence();
+  for (int b = threadIdx.x; b < blocks; b += kBlock) {
+#pragma unroll
+    for (int d = 0; d < N; d++) {
+      lo[d] = fmin(lo[d], __ldcg(&part[(int64_t)b * 2 * N + d]));
+      hi[d] = fmax(hi[d], __ldcg(&part[(int64_t)b * 2 * N + N + d]));
+    }
+  }
+  reduce();
+  if (threadIdx.x == 0) {
+    A.ticket[set] = 0u;
+#pragma unroll
+    for (int d = 0; d < N; d++) {
+      A.out[6 * set + d] = lo[d];
+      A.out[6 * set + N + d] = hi[d];
     }
   }
 }
@@ -1162,40 +1231,37 @@ int scan_exclusive(Handle& h, const int* in, int* out, int64_t m, int* total, in
 template <class T> int set_limits(Handle& h, T* lo, T* hi) {
   // limits over x (and y for two sets): src/internals/CellOperations.jl:262-324
   const int N = h.dim;
-  bool any = false;
-  T glo[3], ghi[3];
+  LimitArgs<T> A;
+  std::memset((void*)&A, 0, sizeof A);
+  int64_t most = 0;
   for (int s = 0; s < h.nsets; s++) {
-    SetData& S = h.sets[s];
-    T slo[3] = {0, 0, 0}, shi[3] = {0, 0, 0};
-    if (S.n > 0) {
-      int nb = std::min<int64_t>(1024, (S.n + kBlock - 1) / kBlock);
-      if (!S.minmax.reserve(sizeof(T) * 2 * N * nb)) return ERR_NOMEM;
-      if (N == 3) k_minmax<T, 3><<<nb, kBlock, 0, h.stream>>>(S.x.as<T>(), (int)S.n, S.minmax.as<T>());
-      else k_minmax<T, 2><<<nb, kBlock, 0, h.stream>>>(S.x.as<T>(), (int)S.n, S.minmax.as<T>());
-      CLM_CUDA_TRY(h, cudaGetLastError());
-    h.launches++;
-      std::vector<T> part((size_t)(2 * N * nb));
-      CLM_CUDA_TRY(h, cudaMemcpyAsync(part.data(), S.minmax.p, part.size() * sizeof(T), cudaMemcpyDeviceToHost, h.stream));
-      CLM_CUDA_TRY(h, cudaStreamSynchronize(h.stream));
-      for (int d = 0; d < N; d++) {
-        slo[d] = part[d];
-        shi[d] = part[N + d];
-      }
-      for (int b = 1; b < nb; b++)
-        for (int d = 0; d < N; d++) {
-          slo[d] = geo::jmin(slo[d], part[(size_t)b * 2 * N + d]);
-          shi[d] = geo::jmax(shi[d], part[(size_t)b * 2 * N + N + d]);
-        }
-    }
-    for (int d = 0; d < N; d++) {
-      glo[d] = any ? geo::jmin(glo[d], slo[d]) : slo[d];
-      ghi[d] = any ? geo::jmax(ghi[d], shi[d]) : shi[d];
-    }
-    any = true;
+    A.x[s] = h.sets[s].x.as<T>();
+    A.n[s] = (int)h.sets[s].n;
+    most = std::max(most, h.sets[s].n);
   }
-  for (int d = 0; d < N; d++) {
-    lo[d] = glo[d];
-    hi[d] = ghi[d];
+  T* out = reinterpret_cast<T*>(h.pres);
+  if (most > 0) {
+    DevBuf& b = h.sets[0].minmax;
+    const void* at = b.p;
+    const size_t parts = sizeof(T) * 2 * 2 * N * kLimitBlocks;
+    if (!b.reserve(parts + 2 * sizeof(unsigned))) return ERR_NOMEM;
+    A.part = b.as<T>();
+    A.ticket = reinterpret_cast<unsigned*>(b.as<char>() + parts);
+    if (b.p != at) CLM_CUDA_TRY(h, cudaMemsetAsync(A.ticket, 0, 2 * sizeof(unsigned), h.stream));
+    A.out = out;
+    const dim3 grid((unsigned)std::min<int64_t>(kLimitBlocks, (most + kBlock - 1) / kBlock), (unsigned)h.nsets);
+    if (N == 3) k_limits<T, 3><<<grid, kBlock, 0, h.stream>>>(A);
+    else k_limits<T, 2><<<grid, kBlock, 0, h.stream>>>(A);
+    CLM_CUDA_TRY(h, cudaGetLastError());
+    h.launches++;
+    CLM_CUDA_TRY(h, cudaStreamSynchronize(h.stream));
+  }
+  for (int s = 0; s < h.nsets; s++) {
+    for (int d = 0; d < N; d++) {
+      const T slo = h.sets[s].n > 0 ? out[6 * s + d] : T(0), shi = h.sets[s].n > 0 ? out[6 * s + N + d] : T(0);
+      lo[d] = s ? geo::jmin(lo[d], slo) : slo;
+      hi[d] = s ? geo::jmax(hi[d], shi) : shi;
+    }
   }
   return OK;
 }
@@ -1218,25 +1284,9 @@ template <class T> int64_t copy_capacity(const SetData& S, const Geometry<T>& g)
   return std::max<int64_t>(std::max<int64_t>(S.copy_cap, (int64_t)est), n + 64);
 }
 
-// One system of few particles: k_build_small.  `launched` says whether it took the build (a device that cannot hold
-// the grid at once leaves it to the counting build).
+// One system of few particles, for k_build_small: the set's buffers and its part of the launch.
 template <class T>
-int build_small(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, int64_t ncells, int64_t cap, bool* launched) {
-  *launched = false;
-  using Kernel = void (*)(const SmallBuild<T>);
-  Kernel k = (N == 3) ? (Kernel)k_build_small<T, 3, kShapeGeneral> : (Kernel)k_build_small<T, 2, kShapeGeneral>;
-  if constexpr (std::is_same<T, double>::value) {
-    if (N == 3 && dg.shape == kShapeDiag) k = k_build_small<T, 3, kShapeDiag>;
-    else if (N == 3 && dg.shape == kShapeUpper) k = k_build_small<T, 3, kShapeUpper>;
-  }
-  static const int sms = [] {
-    int v = 0, dev = 0, coop = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    return coop ? v : 0;
-  }();
-  if (sms <= 0) return OK;
+int prepare_small(Handle& h, SetData& S, int N, int64_t n, int64_t ncells, int64_t cap, SmallSet<T>& B) {
   // the counters of this build and the next, the barrier, and the buckets
   const size_t words = 4 * (size_t)ncells + 2;
   const void* at = S.small_buf.p;
@@ -1253,9 +1303,7 @@ int build_small(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, i
     S.small_epoch = 0;
   }
   S.small_epoch++;
-  SmallBuild<T> B;
   std::memset((void*)&B, 0, sizeof B);
-  B.P.g = dg;
   B.P.x = S.x.as<T>();
   B.P.n = (int)n;
   B.P.wrapped = S.wrapped.as<T>();
@@ -1279,16 +1327,52 @@ int build_small(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, i
   B.off = S.off.as<float4>();
   B.xq = S.xq.as<float4>();
   B.code = S.code.as<int>();
-  void* args[] = {&B};
-  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k, dim3((unsigned)sms), dim3(kSmallThreads), args, 0, h.stream);
-  if (e != cudaSuccess) S.small_cells = 0;
-  if (e == cudaErrorCooperativeLaunchTooLarge) {
+  return OK;
+}
+
+// Blocks of the one-launch build (one per SM); 0 if the device has no cooperative launch.
+inline int small_blocks() {
+  static const int sms = [] {
+    int v = 0, dev = 0, coop = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    return coop && v >= 2 ? v : 0;
+  }();
+  return sms;
+}
+
+// The launch for the sets that were prepared (`count` of them, in A.set[0] and then A.set[1]).
+// `refused`: the device cannot hold the grid at once (a part of it only, for this process).
+template <class T> int launch_small(Handle& h, SmallBuild<T>& A, int count, int N, bool* refused) {
+  using Kernel = void (*)(const SmallBuild<T>);
+  Kernel k = (N == 3) ? (Kernel)k_build_small<T, 3, kShapeGeneral> : (Kernel)k_build_small<T, 2, kShapeGeneral>;
+  if constexpr (std::is_same<T, double>::value) {
+    if (N == 3 && A.g.shape == kShapeDiag) k = k_build_small<T, 3, kShapeDiag>;
+    else if (N == 3 && A.g.shape == kShapeUpper) k = k_build_small<T, 3, kShapeUpper>;
+  }
+  const int blocks = small_blocks();
+  A.split = blocks;
+  if (count == 2) {  // blocks in proportion to the particles, and at least an eighth each
+    const double share = (double)A.set[0].P.n / ((double)A.set[0].P.n + (double)A.set[1].P.n);
+    A.split = std::min(std::max((int)(share * blocks), std::max(1, blocks / 8)), blocks - std::max(1, blocks / 8));
+  }
+  void* args[] = {&A};
+  const cudaError_t e =
+      cudaLaunchCooperativeKernel((const void*)k, dim3((unsigned)blocks), dim3(kSmallThreads), args, 0, h.stream);
+  *refused = e == cudaErrorCooperativeLaunchTooLarge;
+  if (e != cudaSuccess) {
+    for (int s = 0; s < h.nsets; s++) {
+      h.sets[s].small_cells = 0;
+      if (h.sets[s].small) h.sets[s].dirty = true;
+    }
+  }
+  if (*refused) {
     cudaGetLastError();
     return OK;
   }
   CLM_CUDA_TRY(h, e);
   h.launches++;
-  *launched = true;
   return OK;
 }
 
@@ -1423,7 +1507,6 @@ int build_bucket(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, 
   int* max_cell = S.copy_off.as<int>() + n + 1;  // the largest cell
   PlaceArgs<T> P;
   std::memset((void*)&P, 0, sizeof P);
-  P.g = dg;
   P.gtab = h.batch.gtab.as<DevGeom<T>>();
   P.psys = h.batch.psys.as<int>();
   P.cbase = h.batch.cbase_d.as<int>();
@@ -1435,7 +1518,7 @@ int build_bucket(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, 
   P.slots = slots;
   P.cf = cell_cf;
   P.err = err;
-  using Place = void (*)(const PlaceArgs<T>, int*);
+  using Place = void (*)(const DevGeom<T>, const PlaceArgs<T>, int*);
   Place place;
   if (batch) place = (N == 3) ? (Place)k_wrap_place<T, 3, kShapeGeneral, true> : (Place)k_wrap_place<T, 2, kShapeGeneral, true>;
   else place = (N == 3) ? (Place)k_wrap_place<T, 3, kShapeGeneral, false> : (Place)k_wrap_place<T, 2, kShapeGeneral, false>;
@@ -1444,7 +1527,7 @@ int build_bucket(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, 
     if (!batch && N == 3 && dg.shape == kShapeDiag) place = k_wrap_place<T, 3, kShapeDiag, false>;
     else if (!batch && N == 3 && dg.shape == kShapeUpper) place = k_wrap_place<T, 3, kShapeUpper, false>;
   }
-  place<<<(unsigned)((n + WE_BLOCK - 1) / WE_BLOCK), WE_BLOCK, 0, h.stream>>>(P, max_cell);
+  place<<<(unsigned)((n + WE_BLOCK - 1) / WE_BLOCK), WE_BLOCK, 0, h.stream>>>(dg, P, max_cell);
   CLM_CUDA_TRY(h, cudaGetLastError());
   h.launches++;
   k_cell_scan<<<(unsigned)ct, kBlock, 0, h.stream>>>(cell_cf, (int)ncells, S.cell_start.as<int>(), S.cell_flags.as<int>(),
@@ -1457,13 +1540,13 @@ int build_bucket(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, 
   const int most = std::min(kGatherMax / slots, kGatherCells);
   const int per = (int)std::max(1.0, std::min((double)most, 512.0 * (double)ncells / (double)cap));
   const size_t smem = (size_t)per * slots * 9;
-  using Gather = void (*)(const PlaceArgs<T>, const int*, const int*, int, int, int, T*, T*, T*, float4*, float4*, int*,
+  using Gather = void (*)(const DevGeom<T>, const PlaceArgs<T>, const int*, const int*, int, int, int, T*, T*, T*, float4*, float4*, int*,
                           unsigned long long*, int64_t);
   Gather gather;
   if (batch) gather = (N == 3) ? (Gather)k_bucket_gather<T, 3, true> : (Gather)k_bucket_gather<T, 2, true>;
   else gather = (N == 3) ? (Gather)k_bucket_gather<T, 3, false> : (Gather)k_bucket_gather<T, 2, false>;
   gather<<<(unsigned)((ncells + per - 1) / per), kBlock, smem, h.stream>>>(
-      P, h.batch.cell_sys.as<int>(), S.cell_start.as<int>(), (int)ncells, per, (int)cap, S.px.as<T>(), S.py.as<T>(),
+      dg, P, h.batch.cell_sys.as<int>(), S.cell_start.as<int>(), (int)ncells, per, (int)cap, S.px.as<T>(), S.py.as<T>(),
       S.pz.as<T>(), S.off.as<float4>(), S.xq.as<float4>(), S.code.as<int>(), st_c, w_c + w_f);
   CLM_CUDA_TRY(h, cudaGetLastError());
   h.launches++;
@@ -1471,7 +1554,8 @@ int build_bucket(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, 
   return OK;
 }
 
-template <class T> int build_set(Handle& h, int set, const Geometry<T>& g) {
+// `small`: where a set that k_build_small takes leaves its part of the launch (`count` sets so far).
+template <class T> int build_set(Handle& h, int set, const Geometry<T>& g, SmallBuild<T>& small, int& count) {
   SetData& S = h.sets[set];
   const int N = g.dim;
   const int64_t n = S.n;
@@ -1529,11 +1613,14 @@ template <class T> int build_set(Handle& h, int set, const Geometry<T>& g) {
   S.counted = !batch && !crowded;
   S.small = false;
   S.bucket_used = 0;
-  if (!batch && !S.prefer_radix && !S.small_off && n <= kSmallParticles && ncells <= kSmallCells &&
+  if (!batch && small_blocks() > 0 && !S.prefer_radix && !S.small_off && n <= kSmallParticles && ncells <= kSmallCells &&
       copies_expected(S, g) <= kSmallPerCell * (double)ncells) {
-    const int st = build_small<T>(h, S, dg, N, n, ncells, cap, &S.small);
-    if (S.small) S.counted = true;
-    if (st || S.small) return st;
+    small.g = dg;
+    const int st = prepare_small<T>(h, S, N, n, ncells, cap, small.set[count]);
+    if (st) return st;
+    count++;
+    S.small = S.counted = true;
+    return OK;
   }
   double per_cell = (double)n;  // copies per cell at uniform density
   if (!batch)
@@ -1683,6 +1770,31 @@ template <class T> int build_set(Handle& h, int set, const Geometry<T>& g) {
   return OK;
 }
 
+// Builds the sets of `which` (bit s: set s), all enqueued on the handle's stream.
+template <class T> int build_sets(Handle& h, const Geometry<T>& g, unsigned which) {
+  for (bool again = true; again;) {
+    SmallBuild<T> small;
+    int count = 0;
+    for (int s = 0; s < h.nsets; s++) {
+      if (!(which >> s & 1u)) continue;
+      const int st = build_set<T>(h, s, g, small, count);
+      if (st) return st;
+    }
+    again = false;
+    if (count) {
+      const int st = launch_small<T>(h, small, count, g.dim, &again);
+      if (st) return st;
+    }
+    which = 0;  // refused: those sets again, by the other builds
+    for (int s = 0; again && s < h.nsets; s++)
+      if (h.sets[s].small) {
+        h.sets[s].small_off = true;
+        which |= 1u << s;
+      }
+  }
+  return OK;
+}
+
 // Reads the device totals of the last build of every set (after the caller synchronized the stream
 // through `staged`, which the caller filled with enqueue_build_totals) and checks the error word.
 Totals build_totals(Handle& h) {
@@ -1776,8 +1888,8 @@ int check_build_totals(Handle& h, bool* overflow) {
 
 template void fill_devgeom<float>(const Geometry<float>&, int, DevGeom<float>&);
 template void fill_devgeom<double>(const Geometry<double>&, int, DevGeom<double>&);
-template int build_set<float>(Handle&, int, const Geometry<float>&);
-template int build_set<double>(Handle&, int, const Geometry<double>&);
+template int build_sets<float>(Handle&, const Geometry<float>&, unsigned);
+template int build_sets<double>(Handle&, const Geometry<double>&, unsigned);
 template int set_limits<float>(Handle&, float*, float*);
 template int set_limits<double>(Handle&, double*, double*);
 

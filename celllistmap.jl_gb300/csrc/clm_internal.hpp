@@ -200,7 +200,7 @@ constexpr size_t kResultBytes = 256 + 16 * 256 + 128;
 
 // Build (clm_build.cu)
 int scan_exclusive(Handle& h, const int* in, int* out, int64_t m, int* total, int depth = 0);
-template <class T> int build_set(Handle& h, int set, const Geometry<T>& g);
+template <class T> int build_sets(Handle& h, const Geometry<T>& g, unsigned which);
 // Words that a build leaves on the device for the host: the totals of every build not read back yet and the error
 // word, copied to the handle's pinned area by the kernel that ends the call (or by enqueue_build_totals).
 struct Totals {
