@@ -160,14 +160,15 @@ int32_t clm_create(int32_t dtype, int32_t dim, int32_t nsets, clm_handle* out) {
     return ERR_CUDA;
   }
   h->own_stream = true;
-  if (cudaMallocHost((void**)&h->pinned, 256) != cudaSuccess ||
-      cudaMallocHost((void**)&h->pres, clm::kResultBytes) != cudaSuccess || !h->err.reserve(64)) {
+  if (cudaMallocHost((void**)&h->pinned, 256 + clm::kResultBytes + clm::kPinnedForces) != cudaSuccess ||
+      !h->err.reserve(64)) {
     if (h->pinned) cudaFreeHost(h->pinned);
-    if (h->pres) cudaFreeHost(h->pres);
     cudaStreamDestroy(h->stream);
     delete h;
     return ERR_CUDA;
   }
+  h->pres = reinterpret_cast<unsigned char*>(h->pinned) + 256;
+  h->pforces = h->pres + clm::kResultBytes;
   cudaMemset(h->err.p, 0, 64);
   for (auto& e : h->ev) cudaEventCreate(&e);
   *out = h;
@@ -180,7 +181,6 @@ int32_t clm_destroy(clm_handle h) {
   for (auto& e : h->ev)
     if (e) cudaEventDestroy(e);
   if (h->pinned) cudaFreeHost(h->pinned);
-  if (h->pres) cudaFreeHost(h->pres);
   if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
   delete h;
   return OK;

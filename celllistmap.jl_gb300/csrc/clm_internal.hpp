@@ -173,8 +173,9 @@ struct Handle {
   DevBuf partial;    // per-block partial reductions
   DevBuf opbuf;      // operator parameter staging (types, tables, velocities, bins)
   DevBuf outbuf;     // device outputs staged before copying to the caller
-  int* pinned = nullptr;       // small pinned host staging area (256 bytes)
+  int* pinned = nullptr;       // small pinned host staging area (256 bytes), then pres and pforces in one allocation
   unsigned char* pres = nullptr;  // pinned host copy of a map's results (kResultBytes)
+  unsigned char* pforces = nullptr;  // pinned host copy of the forces of a small map (kPinnedForces)
   cudaEvent_t ev[4] = {};
   float build_ms = 0, map_ms = 0;
   bool build_timing_pending = false;
@@ -186,7 +187,11 @@ struct Handle {
 
 // Results of one map on the device: scalar, count, minimum and its pair (first 256 bytes), histogram counts
 // and sums (16 x 256 bytes), adjoint sums.
-constexpr size_t kResultBytes = 256 + 16 * 256 + 128;
+constexpr size_t kResultBytes = 256 + 16 * 256 + 256;
+// Forces up to this size go to the host through pinned memory that the kernel writes, larger ones by a copy to the
+// caller's pageable memory after it: the kernel's stores to the host are the quicker way for 24 KB (1003 particles in
+// Float64: a step of 75.5 us against 80.5), even at 96 KB, and the slower at 240 KB (104.5 us against 98.5).
+constexpr size_t kPinnedForces = 64 * 1024;
 
 // Status helpers
 #define CLM_CUDA_TRY(h, call)                                                            \

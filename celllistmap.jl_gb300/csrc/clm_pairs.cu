@@ -531,6 +531,7 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
   const bool f4 = !(std::is_same<T, double>::value && !A.split);
   T* dst_x = nullptr;
   T* dst_y = nullptr;
+  const bool pinned_forces = forces && !O->out_on_device && sizeof(T) * (nx + ny) * N <= kPinnedForces;
   const size_t acc_bytes = align((f4 ? sizeof(float4) : sizeof(double) * N) * (nx + ny));
   if (forces) {
     if (!h.outbuf.reserve(acc_bytes + sizeof(T) * (nx + ny) * N + 256)) return ERR_NOMEM;
@@ -539,8 +540,8 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
     A.f4x = h.outbuf.as<float4>();
     A.f4y = A.f4x + nx;
     if (!O->out_on_device) {
-      // staged after the accumulators when the caller gave host pointers
-      dst_x = (T*)(h.outbuf.as<char>() + acc_bytes);
+      // the caller gave host pointers: small forces are written to pinned memory, others staged after the accumulators
+      dst_x = pinned_forces ? (T*)h.pforces : (T*)(h.outbuf.as<char>() + acc_bytes);
       dst_y = dst_x + nx * N;
     } else {
       dst_x = (T*)O->forces_x;
@@ -616,13 +617,17 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
     else k_finish<T, 2><<<blocks, kReduce, 0, h.stream>>>(F);
     CLM_CUDA_TRY(h, cudaGetLastError());
     h.launches++;
-    if (forces && !O->out_on_device) {
+    if (forces && !O->out_on_device && !pinned_forces) {
       if (O->forces_x && nx)
         CLM_CUDA_TRY(h, cudaMemcpyAsync(O->forces_x, dst_x, sizeof(T) * nx * N, cudaMemcpyDeviceToHost, h.stream));
       if (O->forces_y && ny)
         CLM_CUDA_TRY(h, cudaMemcpyAsync(O->forces_y, dst_y, sizeof(T) * ny * N, cudaMemcpyDeviceToHost, h.stream));
     }
     CLM_CUDA_TRY(h, cudaStreamSynchronize(h.stream));
+    if (pinned_forces) {
+      if (O->forces_x && nx) std::memcpy(O->forces_x, dst_x, sizeof(T) * nx * N);
+      if (O->forces_y && ny) std::memcpy(O->forces_y, dst_y, sizeof(T) * ny * N);
+    }
     if (opk != OPK_NL) break;
     std::memcpy(&h.nl_n, h.pres + 8, sizeof(h.nl_n));
     if (h.nl_n <= h.nl_cap || attempt == 1) break;
