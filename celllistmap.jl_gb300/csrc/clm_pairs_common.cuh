@@ -146,19 +146,19 @@ template <class T, int N> __device__ __forceinline__ T exact_d2(const T* dx) {
 }
 
 // The exact test of a pair whose FP32 distance is near the cutoff: d2 <= cutoff^2, and the reference's
-// projection filter near the cutoff, seen from the cell of the reference's i (the candidate's cell is `me` away;
+// projection filter above proj_lo, seen from the cell of the reference's i (the candidate's cell is `me` away;
 // `same`: the particle's own cell, where the filter does not apply; swapped: the candidate is the
 // reference's i).  A call: a few pairs in ten thousand come here, and its registers stay out of the sweep.
 template <class T, int N>
-__device__ __noinline__ bool near_cutoff(const DevGeom<T>& g, T cutoff_sqr, float thr_lo, int3 ci, int me, bool same,
-                                         bool swapped, T x0, T x1, T x2, T y0, T y1, T y2) {
+__device__ __noinline__ bool near_cutoff(const DevGeom<T>& g, T cutoff_sqr, int3 ci, int me, bool same, bool swapped, T x0,
+                                         T x1, T x2, T y0, T y1, T y2) {
   const T xi[3] = {x0, x1, x2}, xj[3] = {y0, y1, y2};
   T dx[3];
 #pragma unroll
   for (int d = 0; d < N; d++) dx[d] = xsub(xi[d], xj[d]);
   const T d2 = exact_d2<T, N>(dx);
   if (!nonneg_le(d2, cutoff_sqr)) return false;
-  if (!nonneg_lt((T)thr_lo, d2) || same) return true;
+  if (!nonneg_lt(g.proj_lo, d2) || same) return true;
   const int ca[3] = {ci.x, ci.y, ci.z};
   const int cj[3] = {ci.x + (me & 255) - 128, ci.y + ((me >> 8) & 255) - 128,
                      (N == 3) ? ci.z + ((me >> 16) & 255) - 128 : 1};

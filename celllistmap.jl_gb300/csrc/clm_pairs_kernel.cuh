@@ -488,11 +488,11 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
               const int3 c3 = make_int3(ci[0], ci[1], ci[2]);
               if constexpr (FP64) {
                 if constexpr (!EXACT64) load_x(jp, ie, q);
-                return near_cutoff<T, N>(gc, g.cutoff_sqr, g.thr_lo, c3, W.meta[lo], e < same_end, sw, q.xi[0], q.xi[1],
+                return near_cutoff<T, N>(gc, g.cutoff_sqr, c3, W.meta[lo], e < same_end, sw, q.xi[0], q.xi[1],
                                          (N == 3) ? q.xi[2] : T(0), q.xj[0], q.xj[1], (N == 3) ? q.xj[2] : T(0));
               } else {
                 q.d2f = exact_d2<float, N>(q.dvf);
-                return near_cutoff<T, N>(gc, g.cutoff_sqr, g.thr_lo, c3, W.meta[lo], e < same_end, sw, p4.x, p4.y, p4.z,
+                return near_cutoff<T, N>(gc, g.cutoff_sqr, c3, W.meta[lo], e < same_end, sw, p4.x, p4.y, p4.z,
                                          W.p[0][jp], W.p[1][jp], (N == 3) ? W.p[2][jp] : 0.f);
               }
             }

@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 4) ? 6 : 5)
                       d2 = exact_d2<T, N>(dxs);
                       const int run_q = jp / kPad;
                       const int e = w0 + ((run_q >> GS) << (5 + GS)) + ((jp - run_q * kPad) << GS) + (run_q & ((1 << GS) - 1));
-                      hit = near_cutoff<T, N>(gc, g.cutoff_sqr, g.thr_lo, make_int3(ci[0], ci[1], ci[2]),
+                      hit = near_cutoff<T, N>(gc, g.cutoff_sqr, make_int3(ci[0], ci[1], ci[2]),
                                               W.meta[W.entry_of(e)], e < same_end, sw, xi[0], xi[1], xi[2], xj[0], xj[1],
                                               xj[2]);
                     }
