@@ -90,6 +90,7 @@ template <class T> struct PairArgs {
   // work decomposition and batches of independent systems
   int cell_split;               // parts of a cell's particles: part p takes the chunks p, p + S, p + 2S, ... of 32
   int stage_split;              // parts of its candidates: part p takes the stages p, p + S, p + 2S, ...
+  int part_step;                // turn of a cell's parts per wave of items (part_of)
   int stage;                    // candidates per stage, at most kStage (a multiple of 32)
   float hist_err;               // RHIST, Float64 exact: absolute error of the FP32 distance of cell offsets
   const DevGeom<T>* gtab;       // batch: geometry of each system

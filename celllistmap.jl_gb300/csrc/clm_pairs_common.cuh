@@ -137,6 +137,18 @@ __device__ __forceinline__ void force_add(const PairArgs<T>& A, bool ys, int idx
   }
 }
 
+// The part of its cell that work item r is, the cell being the rcell-th of S parts each.  The parts of a cell differ in
+// size (the first stages hold the cell itself, the last are short), and a warp takes every nw-th item: in plain order a
+// warp whose nw is a multiple of S would take the same part of every cell.  So the parts of a cell are turned by `step`
+// (A.part_step, such that nw + step and S have no common factor) for each wave of items before it.  The neighbour list
+// of 100k Float64 points at cutoff 8 (8 parts per cell, 3040 warps): map 690 -> 625 us.
+__device__ __forceinline__ int part_of(int r, int rcell, int S, int nw, int step) {
+  const int first = rcell * S;
+  unsigned p = (unsigned)(r - first);
+  if (step) p = (p + (unsigned)(first / nw) * (unsigned)step) % (unsigned)S;
+  return (int)p;
+}
+
 // The reference's d2, with its separately rounded operations.
 template <class T, int N> __device__ __forceinline__ T exact_d2(const T* dx) {
   T d2 = xmul(dx[0], dx[0]);

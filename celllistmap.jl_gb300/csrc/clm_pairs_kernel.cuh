@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
     int rcell = r, part_i = 0, part_j = 0;
     if (S > 1) {
       rcell = r / S;
-      part_i = r - rcell * S;
+      part_i = part_of(r, rcell, S, nw, A.part_step);
       part_j = part_i / SI;
       part_i -= part_j * SI;
     }
@@ -988,6 +988,19 @@ inline int resident_grid(int want, int per_sm) {
   return std::max(1, std::min(want, std::max(1, per_sm) * sms));
 }
 
+// The smallest step with no common factor of n + step and parts.
+inline int coprime_step(int n, int parts) {
+  for (int step = 0;; step++) {
+    int a = n + step, b = parts;
+    while (b) {
+      const int t = a % b;
+      a = b;
+      b = t;
+    }
+    if (a == 1) return step;
+  }
+}
+
 template <class T, int N, int OPK, bool SPLIT, bool CROSS, bool BATCH = false, int OPC = 0>
 cudaError_t launch_k(int& grid, cudaStream_t st, const PairArgs<T>& A) {
   using FA = typename std::conditional<std::is_same<T, double>::value && !SPLIT, double, float>::type;
@@ -1009,7 +1022,15 @@ cudaError_t launch_k(int& grid, cudaStream_t st, const PairArgs<T>& A) {
       per_sm = std::min(per_sm, sizeof(T) == 4 ? kAdjBlocks32 : kAdjBlocks64);
   }
   grid = resident_grid(grid, per_sm);
-  k<<<grid, kThreads, dyn, st>>>(A);
+  // turned parts (part_of), except where the order of the sums has to stay
+  const int parts = A.cell_split * A.stage_split;
+  if (!BATCH && parts > 1 && !in_rounds(OPK, sizeof(T) == 8, SPLIT, BATCH)) {
+    PairArgs<T> B = A;
+    B.part_step = coprime_step(grid * kWarps, parts);
+    k<<<grid, kThreads, dyn, st>>>(B);
+  } else {
+    k<<<grid, kThreads, dyn, st>>>(A);
+  }
   return cudaGetLastError();
 }
 
