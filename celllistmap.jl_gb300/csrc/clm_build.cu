@@ -4,25 +4,26 @@
 // of add_particles! 940-950 and add_particle_to_celllist! 983-1057) and the
 // non-periodic build (src/internals/NonPeriodicCells.jl:93-251).
 //
-// One system of at most 2^16 particles: k_build_small, the whole build in one cooperative launch.
-// One larger system (counting build, four launches after one memset):
-//   k_wrap_stage    wrap into the first cell (wrap_to_first, CellOperations.jl:91-94),
+// One system of at most 2^16 particles: k_build_small, the whole build in one cooperative launch (both sets of an x-y
+// handle together).
+// Larger systems and batches (bucket build, three launches):
+//   k_wrap_place    wrap into the first cell (wrap_to_first, CellOperations.jl:91-94),
 //                   rotate, test the 3^N-1 translation images against the computing
-//                   box (replicate_particle!, Box.jl:556-566), stage one (cell,
-//                   particle<<5|image) key/value per copy (particle_cell +
-//                   real_particle_border_case) in the tile's slots, and count the
-//                   copies of every cell (atomic adds)
+//                   box (replicate_particle!, Box.jl:556-566), find the cell of each copy
+//                   (particle_cell + real_particle_border_case) and give it a place in its
+//                   cell's bucket
 //   k_cell_scan     cell starts and the list of cells that contain real particles
-//   k_cell_scatter  copies to their cells' slots in arrival order (atomic cursors)
-//   k_rank_gather   each copy to its rank by value inside its cell (particle-index
+//   k_bucket_gather each copy to its rank by value inside its cell (particle-index
 //                   order, the reference's serial order), with its coordinates (SoA),
 //                   particle code and 16-byte candidate record
-// One system with crowded cells (more than kCountingMaxPerCell copies per cell
-// expected): k_wrap_emit without the counters, a stable LSD radix sort of the keys by
-// cell, k_gather (cell starts from the sorted keys) and k_compact_1pass.
-// Batches (global cell index over all systems): k_wrap_count_b, a scan of the
-// copies, k_emit_b, the radix sort, k_gather_b, and the real-cell scan and
-// compaction.
+// One system with a cell too full for a bucket (counting build): k_wrap_stage stages one
+// (cell, particle<<5|image) key/value per copy and counts the copies of every cell,
+// k_cell_scan, k_cell_scatter (copies to their cells in arrival order), k_rank_gather.
+// Crowded cells (more than kCountingMaxPerCell copies per cell expected, or more than
+// kRadixAbovePerCell met): k_wrap_emit, a stable LSD radix sort of the keys by
+// cell, k_gather (cell starts from the sorted keys) and k_compact_1pass; batches:
+// k_wrap_count_b, a scan of the copies, k_emit_b, the radix sort, k_gather_b, and the
+// real-cell scan and compaction.
 //
 // Every kernel bounds-checks its indices; inconsistencies set bits of the
 // handle's device error word instead of faulting.
@@ -407,7 +408,7 @@ __global__ void __launch_bounds__(WE_BLOCK) k_wrap_emit(DevGeom<T> g, const T* _
   }
 }
 
-// One system, counting build: the same wrap, image tests and keys, with the copies of each tile of
+// One system, counting build (cells too full for a bucket): the same wrap, image tests and keys, with the copies of each tile of
 // WE_BLOCK particles in the tile's own range of `slots` staging slots (the in-cell ranking orders a cell by
 // value, so the copies need no position in particle order, and no tile waits on an earlier one).  Each
 // tile writes its number of copies; a tile with more copies than slots writes none and flags
@@ -624,7 +625,11 @@ __global__ void __launch_bounds__(kBlock) k_rank_gather(DevGeom<T> g, const T* _
 //
 // A warp's copies are shared out evenly over its block before their cells are computed: most particles have one
 // copy, a few have seven, and lanes that walked their own would leave the others idle (and in Float64 hold the FP64
-// pipe, 16 cycles per warp instruction, for each round).
+// pipe, 16 cycles per warp instruction, for each round: 106 FP64 instructions per warp of 256,000 Lennard-Jones
+// particles in a sheared cell, now 72).
+// Builds against the counting build's four kernels: 1M Float32 81 us (91), 256,000 Float64 77 (93), 100,000 Float64 42
+// (57), 200,000 Float32 39 (45); 1,024 systems of 200 to 2,000 against the radix sort: 360 us (530).  What bounds
+// it: Float32 issue and latency (2.5 warp instructions per cycle), Float64 the FP64 queue (pipe 62 to 75 % busy).
 template <class T> struct PlaceArgs {
   const DevGeom<T>* gtab;  // batches: geometry per system, system of each particle, first cell of each system
   const int* psys;
@@ -822,10 +827,10 @@ __global__ void __launch_bounds__(kBlock) k_bucket_gather(const __grid_constant_
 // (DERR_TILE_OVERFLOW) and the set is built by the other kernels from then on.
 constexpr int kSmallThreads = 512;
 constexpr int kBucket = 128;
-// Up to here the one launch is clearly the shorter build (GB300, Float32 / Float64 at liquid density: 4,000
-// particles 25 / 31 us against 37 / 43, 32,000 27 / 35 against 40 / 46, 64,000 30 / 40 against 39 / 50).  At 128,000
-// it still is, 40 / 57 against 46 / 65, but its blocks wait for a whole free device, which costs a program that
-// keeps other streams busy more than that; at 400,000 it is not (70 / 114 against 62 / 109).
+// Up to here the one launch is clearly the shorter build (GB300, Float32 / Float64 at liquid density, against the
+// bucket build: 4,000 particles 18 / 21 us against 28 / 33, 32,000 22 / 27 against 30 / 35, 64,000 26 / 36 against
+// 31 / 41).  At 96,000 they are even (32 / 43 against 33 / 44), and its blocks wait for a whole free device; at 400,000
+// it is the longer one (68 / 108 against 47 / 77).
 constexpr int64_t kSmallParticles = 1 << 16;
 constexpr int64_t kSmallCells = 1 << 15;
 constexpr double kSmallPerCell = 64.0;  // copies per cell expected at uniform density: half a bucket
