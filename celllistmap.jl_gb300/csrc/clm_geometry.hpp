@@ -329,6 +329,17 @@ template <class T> double split_distance_error(const Geometry<T>& g) {
   return std::sqrt((double)g.dim) * (3.0 * g.lcell + 5.0) * cs * std::ldexp(1.0, -24);
 }
 
+// The same with what the float pairs behind the offsets lose far from the origin: a coordinate and a cell origin, each
+// carried in 48 bits, and the differences of their low parts come to less than 64 far 2^-48 per copy and component (far:
+// the largest coordinate of the computing box), more than the bound above once far exceeds some 10^6 cell sides (a
+// non-periodic system around 10^9: 3.6e-6 where the bound above is 6e-7).
+template <class T> double offset_distance_error(const Geometry<T>& g) {
+  double far = 0.0;
+  for (int i = 0; i < g.dim; i++)
+    far = std::max(far, std::max(std::fabs((double)g.cbmin[i]), std::fabs((double)g.cbmax[i])));
+  return split_distance_error(g) + std::sqrt((double)g.dim) * 2.0 * 64.0 * far * std::ldexp(1.0, -48);
+}
+
 // The split-form radial histogram decides bins from that FP32 distance and re-decides exactly within 2^-12
 // (relative) of an edge, which covers the error for every edge above split_distance_error * 2^12.  True when
 // all positive edges are above it (the bins then equal the exact form's).  An edge at 0 only separates

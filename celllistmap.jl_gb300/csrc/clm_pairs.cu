@@ -346,7 +346,7 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
   A.cell_split = split.si;
   A.stage_split = split.sj;
   A.stage = split.stage;
-  A.hist_err = (float)(split_distance_error(g) * 1.001);
+  A.hist_err = (float)(offset_distance_error(g) * 1.001);
   const LaunchSel sel{N, opk, A.self != 0, A.split != 0, false};
   const double c_default = (double)g.cutoff;
   {
