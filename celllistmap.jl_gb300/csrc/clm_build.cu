@@ -930,7 +930,9 @@ __global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_cons
     }
     __syncthreads();
   }
-  const bool skip = (__ldcg(B.P.err) & (DERR_TILE_OVERFLOW | DERR_NAN)) != 0;  // the cell list is not used
+  // An overflow: nothing maps this list.  A NaN particle has no copies, and what the others have is gathered all the
+  // same: the map that was enqueued behind this build runs over the list, and the other set's list stays in use.
+  const bool skip = (__ldcg(B.P.err) & DERR_TILE_OVERFLOW) != 0;
   for (int cb = c0; cb < c1; cb += kSmallThreads) {  // 512 cells at a time
     const int c = cb + threadIdx.x;
     int2 v = make_int2(0, 0);
