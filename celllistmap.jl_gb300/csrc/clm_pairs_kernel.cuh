@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
               }
               __syncwarp();
               // The queue is first reduced to the pairs the reference keeps (in place: an entry moves to an
-              // earlier or its own slot, after every lane has read its entry), so that one atomic per sweep
+              // earlier or its own slot), so that one atomic per sweep
               // reserves their places in the list: an atomic on one address takes 0.67 ns on GB300 wherever it
               // comes from, and one per 32 entries took half of the list's time (674 us for 1.07e7 Float64 pairs)
               int kept = 0;
@@ -562,6 +562,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
                   keep = keep_pair(ent & 511, ent >> 9, W.i4[ent >> 9], q);
                 }
                 const unsigned bal = __ballot_sync(FULL, keep);
+                __syncwarp();  // every lane has read its entry (a ballot orders no memory)
                 if (keep) W.q[kept + __popc(bal & ((1u << lane) - 1u))] = (unsigned short)ent;
                 kept += __popc(bal);
                 __syncwarp();
@@ -599,6 +600,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
             }
           } else {
             // ---- sweep: lane t takes the hits t per .. t per + per - 1
+            __syncwarp();  // the masks of all lanes are written (reductions and shuffles order no memory)
             const int per = (H + 31) >> 5;
             const int first = lane * per;
             int left = min(per, H - first);  // this lane's hits (<= 0: none)
