@@ -131,10 +131,7 @@ int build_dispatch(Handle& h, bool sync = true) {
 // and its error bits unread: the next call rebuilds it instead of trusting it.
 void drop_unchecked_builds(Handle& h) {
   for (int s = 0; s < h.nsets; s++) {
-    if (h.sets[s].pending) {
-      h.sets[s].pending = false;
-      h.sets[s].dirty = true;
-    }
+    if (h.sets[s].pending) drop_build(h.sets[s]);
   }
 }
 

@@ -1303,26 +1303,22 @@ int prepare_small(Handle& h, SetData& S, int N, int64_t n, int64_t ncells, int64
       !S.off.reserve(std::is_same<T, float>::value ? 16 : sizeof(float4) * cap) || !S.code.reserve(sizeof(int) * cap) ||
       !S.xq.reserve(std::is_same<T, float>::value ? sizeof(float4) * cap : 16))
     return ERR_NOMEM;
-  if (S.small_cells != ncells || S.small_buf.p != at) {
-    S.small_cells = 0;
+  if (small_needs_clear(S, ncells, S.small_buf.p != at))
     CLM_CUDA_TRY(h, cudaMemsetAsync(S.small_buf.p, 0, sizeof(int) * words, h.stream));
-    S.small_cells = ncells;
-    S.small_epoch = 0;
-  }
-  S.small_epoch++;
+  const int half = small_half(S);
   std::memset((void*)&B, 0, sizeof B);
   B.P.x = S.x.as<T>();
   B.P.n = (int)n;
   B.P.wrapped = S.wrapped.as<T>();
   B.P.bucket = S.small_buf.as<uint32_t>() + words;
   B.P.slots = kBucket;
-  B.P.cf = S.small_buf.as<int>() + ((S.small_epoch & 1) ? 2 * ncells : 0);
+  B.P.cf = S.small_buf.as<int>() + 2 * ncells * half;
   B.P.err = h.err.as<int>();
   B.ncells = (int)ncells;
   B.cap = (int)cap;
-  B.cf_next = S.small_buf.as<int>() + ((S.small_epoch & 1) ? 0 : 2 * ncells);
+  B.cf_next = S.small_buf.as<int>() + 2 * ncells * (1 - half);
   B.bar = reinterpret_cast<unsigned*>(S.small_buf.as<int>() + 4 * ncells);
-  B.epoch = S.small_epoch;
+  B.epoch = S.small_epoch + 1;
   B.cell_start = S.cell_start.as<int>();
   B.cell_flags = S.cell_flags.as<int>();
   B.real_list = S.real_list.as<int>();
@@ -1349,9 +1345,9 @@ inline int small_blocks() {
   return sms;
 }
 
-// The launch for the sets that were prepared (`count` of them, in A.set[0] and then A.set[1]).
+// The launch for the sets that were prepared (`which`; `count` of them, in A.set[0] and then A.set[1]).
 // `refused`: the device cannot hold the grid at once (a part of it only, for this process).
-template <class T> int launch_small(Handle& h, SmallBuild<T>& A, int count, int N, bool* refused) {
+template <class T> int launch_small(Handle& h, SmallBuild<T>& A, unsigned which, int count, int N, bool* refused) {
   using Kernel = void (*)(const SmallBuild<T>);
   Kernel k = (N == 3) ? (Kernel)k_build_small<T, 3, kShapeGeneral> : (Kernel)k_build_small<T, 2, kShapeGeneral>;
   if constexpr (std::is_same<T, double>::value) {
@@ -1368,12 +1364,8 @@ template <class T> int launch_small(Handle& h, SmallBuild<T>& A, int count, int 
   const cudaError_t e =
       cudaLaunchCooperativeKernel((const void*)k, dim3((unsigned)blocks), dim3(kSmallThreads), args, 0, h.stream);
   *refused = e == cudaErrorCooperativeLaunchTooLarge;
-  if (e != cudaSuccess) {
-    for (int s = 0; s < h.nsets; s++) {
-      h.sets[s].small_cells = 0;
-      if (h.sets[s].small) h.sets[s].dirty = true;
-    }
-  }
+  for (int s = 0; s < h.nsets; s++)
+    if (which >> s & 1u) small_launched(h.sets[s], h.sets[s].ncells, e == cudaSuccess);
   if (*refused) {
     cudaGetLastError();
     return OK;
@@ -1778,28 +1770,34 @@ template <class T> int build_set(Handle& h, int set, const Geometry<T>& g, Small
 }
 
 // Builds the sets of `which` (bit s: set s), all enqueued on the handle's stream.
-template <class T> int build_sets(Handle& h, const Geometry<T>& g, unsigned which) {
+template <class T> int enqueue_builds(Handle& h, const Geometry<T>& g, unsigned which) {
   for (bool again = true; again;) {
     SmallBuild<T> small;
     int count = 0;
+    unsigned in_small = 0;
     for (int s = 0; s < h.nsets; s++) {
       if (!(which >> s & 1u)) continue;
-      const int st = build_set<T>(h, s, g, small, count);
+      const int before = count, st = build_set<T>(h, s, g, small, count);
       if (st) return st;
+      if (count > before) in_small |= 1u << s;
     }
     again = false;
     if (count) {
-      const int st = launch_small<T>(h, small, count, g.dim, &again);
+      const int st = launch_small<T>(h, small, in_small, count, g.dim, &again);
       if (st) return st;
     }
-    which = 0;  // refused: those sets again, by the other builds
-    for (int s = 0; again && s < h.nsets; s++)
-      if (h.sets[s].small) {
-        h.sets[s].small_off = true;
-        which |= 1u << s;
-      }
+    which = again ? in_small : 0;  // refused: those sets again, by the other builds
+    for (int s = 0; s < h.nsets; s++)
+      if (which >> s & 1u) h.sets[s].small_off = true;
   }
   return OK;
+}
+// When one fails, none of them counts as built: a set that was only prepared for the joint launch was not.
+template <class T> int build_sets(Handle& h, const Geometry<T>& g, unsigned which) {
+  const int st = enqueue_builds<T>(h, g, which);
+  for (int s = 0; st && s < h.nsets; s++)
+    if (which >> s & 1u) drop_build(h.sets[s]);
+  return st;
 }
 
 // Reads the device totals of the last build of every set (after the caller synchronized the stream

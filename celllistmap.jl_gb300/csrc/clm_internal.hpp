@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "clm_device.cuh"
+#include "clm_build_state.hpp"
 #include "clm_geometry.hpp"
 
 namespace clm {
@@ -60,10 +61,8 @@ struct DevBuf {
 };
 
 // One particle set and its cell list on the device.
-struct SetData {
+struct SetData : BuildState {
   int64_t n = 0;
-  bool dirty = true;
-  bool built = false;
   DevBuf x;                 // positions as given (n x dim, column-major dim x n)
   DevBuf wrapped;           // wrapped (and rotated) positions, n x dim
   DevBuf mask;              // per particle: bit k set if image k lies in the computing box
@@ -83,7 +82,6 @@ struct SetData {
   int64_t n_real_cells = 0;
   int64_t copy_cap = 0;      // capacity for copies learned from previous builds
   int64_t cap_used = 0;      // capacity used by the last build
-  bool pending = false;      // the device totals of the last build were not read back yet
   bool counted = false;      // the last build was the counting build (its largest cell is read back)
   bool prefer_radix = false; // a counting build met a cell of more than kRadixAbovePerCell copies
   int tile_mult = 0;         // counting build: staging slots per particle of a tile (0: from the estimate)
@@ -91,8 +89,6 @@ struct SetData {
   int64_t ncells = 0;
   // build of a few particles in one launch (k_build_small)
   DevBuf small_buf;          // two sets of per-cell counters, the grid barrier, each cell's copies in arrival order
-  int64_t small_cells = 0;   // cells that it is laid out and cleared for (0: none)
-  unsigned small_epoch = 0;  // launches since then
   bool small = false;        // the last build was one
   bool small_off = false;    // one met a cell with more copies than a bucket holds
   // larger sets and batches: a bucket per cell (k_wrap_place)
