@@ -354,7 +354,6 @@ constexpr int WE_PPT = 1;
 // uniform-density estimate misses) is built by radix from then on: the in-cell ranking costs a cell's size
 // per copy, the radix sort does not depend on it.
 constexpr double kCountingMaxPerCell = 64.0;
-constexpr int kRadixAbovePerCell = 1024;
 constexpr int WE_BLOCK = 256;  // threads (particles) per tile of the wrap kernel
 constexpr int WE_TILE = WE_BLOCK * WE_PPT;
 
@@ -1472,7 +1471,6 @@ int build_counting(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n
 // cell, `densest` the same in the densest system of a batch: seven standard deviations of a Poisson count above it, so
 // that uniform sets never overflow.  Cells of more than 64 copies (their ranks cost a cell's size per copy) and grids
 // of mostly empty cells (the buckets would take more memory than the copies) go to the other builds.
-constexpr int kBucketMost = 256;
 template <class T> int bucket_slots(const SetData& S, double e, double densest, int64_t ncells, int64_t cap) {
   if (S.bucket_off || S.prefer_radix || !(e <= kCountingMaxPerCell) || !(densest < (double)kBucketMost)) return 0;
   const int slots = std::max(S.bucket, ((int)(densest + 7.0 * std::sqrt(densest) + 8.0) + 7) / 8 * 8);
@@ -1831,64 +1829,11 @@ int enqueue_build_totals(Handle& h) {
 }
 
 int check_build_totals(Handle& h, bool* overflow) {
-  *overflow = false;
-  const int errw = h.pinned[40];
-  if (errw & DERR_NAN) {
-    for (int s = 0; s < h.nsets; s++) h.sets[s].dirty = true;
-    h.last_error = "Invalid coordinates found (NaN) in the particle positions.";
-    return ERR_NAN;
-  }
-  for (int s = 0; s < h.nsets; s++) {
-    SetData& S = h.sets[s];
-    if (!S.pending) continue;
-    if (h.pinned[32 + 2 * s] < 0) {  // the 32-bit copy-offset scan wrapped: more than 2^31 - 1 copies
-      S.pending = false;
-      S.dirty = true;
-      h.last_error = "too many particle copies for one set (particles and their periodic images exceed 2^31 - 1)";
-      return ERR_ARG;
-    }
-    S.n_copies = h.pinned[32 + 2 * s];
-    S.n_real_cells = h.pinned[33 + 2 * s];
-    if (S.counted && h.pinned[44 + s] > kRadixAbovePerCell) S.prefer_radix = true;
-    if (S.small && (errw & DERR_TILE_OVERFLOW)) {
-      // a cell had more copies than its bucket: the counting build (or radix, when it finds the cell crowded)
-      S.small_off = S.bucket_off = true;
-      S.dirty = true;
-      *overflow = true;
-    } else if (S.bucket_used && (errw & DERR_TILE_OVERFLOW)) {
-      // more places than the largest cell's copies, or the other builds
-      const int most = h.pinned[44 + s], want = (most + most / 4 + 7) / 8 * 8;
-      if (most > S.bucket_used) {
-        if (want <= kBucketMost) S.bucket = want;
-        else S.bucket_off = true;
-      }
-      S.dirty = true;
-      *overflow = true;
-    } else if (S.counted && (errw & DERR_TILE_OVERFLOW)) {
-      // a tile had more copies than its staging slots: more slots per particle, and build again
-      S.tile_mult = std::min(27, 2 * S.tile_mult);
-      S.dirty = true;
-      *overflow = true;
-    }
-    S.pending = false;
-    if (S.n_copies > S.cap_used || (errw & DERR_COPY_OVERFLOW)) {
-      S.copy_cap = S.n_copies + S.n_copies / 8 + 1024;
-      S.dirty = true;
-      *overflow = true;
-    } else if (S.n_copies > S.copy_cap) {
-      S.copy_cap = S.n_copies;
-    }
-  }
-  if (errw & DERR_SCAN) {
-    for (int s = 0; s < h.nsets; s++) h.sets[s].small_cells = 0;  // a barrier left half open is cleared
-    h.last_error = "cell-list build: a scan tile gave up waiting for an earlier tile";
-    return ERR_INTERNAL;
-  }
-  if (!*overflow && (errw & DERR_CELL_RANGE)) {
-    h.last_error = "cell-list build consistency check failed (particle outside the computing box)";
-    return ERR_INTERNAL;
-  }
-  return OK;
+  BuildState* sets[2] = {&h.sets[0], &h.sets[1]};
+  const BuildCheck c = check_builds(sets, h.nsets, h.pinned);
+  *overflow = c.overflow;
+  if (c.status) h.last_error = c.msg;
+  return c.status;
 }
 
 template void fill_devgeom<float>(const Geometry<float>&, int, DevGeom<float>&);

@@ -2,14 +2,42 @@
 // buffers and launches that they govern (so that the CPU tests run them without a GPU).
 #pragma once
 
+#include <algorithm>
+#include <cstddef>
 #include <cstdint>
 
+#include "clm_device.cuh"
+
 namespace clm {
+
+enum Status {
+  RERUN_BUILD = -1,  // internal: the copies overflowed the capacity; rebuild with the exact size and rerun
+  OK = 0, ERR_ARG = 1, ERR_CELL_TOO_SMALL = 2, ERR_NAN = 3, ERR_DIM = 4, ERR_CUDA = 5, ERR_CAPACITY = 6,
+  ERR_STATE = 7, ERR_TIMEOUT = 8, ERR_NOMEM = 9, ERR_LCELL = 10, ERR_NONPERIODIC_CELL = 11, ERR_INTERNAL = 12
+};
+
+// Cells of more copies than this are built by radix (the counting build ranks each copy against its cell).
+constexpr int kRadixAbovePerCell = 1024;
+// The most places per cell that the bucket build takes.
+constexpr int kBucketMost = 256;
 
 struct BuildState {
   bool dirty = true;
   bool built = false;
   bool pending = false;      // the device totals of the last build were not read back yet
+  int64_t n_copies = 0;      // valid once the build was synchronized (pending == false)
+  int64_t n_real_cells = 0;
+  int64_t copy_cap = 0;      // capacity for copies learned from previous builds
+  int64_t cap_used = 0;      // capacity used by the last build
+  bool counted = false;      // the last build counted its cells' copies (their number and its largest cell are read back)
+  bool prefer_radix = false; // one met a cell of more than kRadixAbovePerCell copies
+  int tile_mult = 0;         // counting build: staging slots per particle of a tile (0: from the estimate)
+  size_t cell_count_zero = 0;  // bytes of the scan words and counters left cleared by the last build (0: clear before use)
+  bool small = false;        // the last build was k_build_small
+  bool small_off = false;    // one met a cell with more copies than a bucket holds
+  int bucket_used = 0;       // bucket build: places per cell of the last build (0: another build)
+  int bucket = 0;            // places that an earlier build's largest cell called for
+  bool bucket_off = false;   // one met a cell with more copies than a bucket may hold
   // k_build_small: two halves of per-cell counters.  A launch counts in one half and clears the other for the next.
   int64_t small_cells = 0;   // cells that they are laid out and cleared for (0: none)
   unsigned small_epoch = 0;  // launches since they were cleared
@@ -36,6 +64,77 @@ inline void small_launched(BuildState& S, int64_t ncells, bool ok) {
 inline void drop_build(BuildState& S) {
   S.pending = false;
   S.dirty = true;
+}
+
+struct BuildCheck {
+  int status;
+  bool overflow;    // the builds are repeated with larger capacities
+  const char* msg;  // of an error status
+};
+
+// After the host has the words of the last builds: `words` is the pinned area that build_totals fills (number of copies
+// of set s at 32 + 2 s, of real cells at 33 + 2 s, the largest cell's copies at 44 + s, the error word at 40).
+inline BuildCheck check_builds(BuildState* const* sets, int nsets, const int* words) {
+  BuildCheck r{OK, false, nullptr};
+  const int errw = words[40];
+  if (errw & DERR_SCAN) {
+    // blocks that gave up waiting left cells unwritten, and words that a later build would find cleared
+    for (int s = 0; s < nsets; s++) {
+      sets[s]->small_cells = 0;
+      sets[s]->cell_count_zero = 0;
+    }
+  }
+  if (errw & DERR_NAN) {
+    for (int s = 0; s < nsets; s++) sets[s]->dirty = true;
+    return {ERR_NAN, false, "Invalid coordinates found (NaN) in the particle positions."};
+  }
+  for (int s = 0; s < nsets; s++) {
+    BuildState& S = *sets[s];
+    if (!S.pending) continue;
+    if (words[32 + 2 * s] < 0) {  // the 32-bit copy-offset scan wrapped: more than 2^31 - 1 copies
+      drop_build(S);
+      return {ERR_ARG, r.overflow,
+              "too many particle copies for one set (particles and their periodic images exceed 2^31 - 1)"};
+    }
+    S.n_copies = words[32 + 2 * s];
+    S.n_real_cells = words[33 + 2 * s];
+    if (S.counted && words[44 + s] > kRadixAbovePerCell) S.prefer_radix = true;
+    if (S.small && (errw & DERR_TILE_OVERFLOW)) {
+      // a cell had more copies than its bucket: the counting build (or radix, when it finds the cell crowded)
+      S.small_off = S.bucket_off = true;
+      S.dirty = true;
+      r.overflow = true;
+    } else if (S.bucket_used && (errw & DERR_TILE_OVERFLOW)) {
+      // more places than the largest cell's copies, or the other builds
+      const int most = words[44 + s], want = (most + most / 4 + 7) / 8 * 8;
+      if (most > S.bucket_used) {
+        if (want <= kBucketMost) S.bucket = want;
+        else S.bucket_off = true;
+      }
+      S.dirty = true;
+      r.overflow = true;
+    } else if (S.counted && (errw & DERR_TILE_OVERFLOW)) {
+      // a tile had more copies than its staging slots: more slots per particle, and build again
+      S.tile_mult = std::min(27, 2 * S.tile_mult);
+      S.dirty = true;
+      r.overflow = true;
+    }
+    S.pending = false;
+    if (S.n_copies > S.cap_used || (errw & DERR_COPY_OVERFLOW)) {
+      S.copy_cap = S.n_copies + S.n_copies / 8 + 1024;
+      S.dirty = true;
+      r.overflow = true;
+    } else if (S.n_copies > S.copy_cap) {
+      S.copy_cap = S.n_copies;
+    }
+  }
+  // A list that a failed build left is not used by a later call: the sets are built again.
+  const bool scan = errw & DERR_SCAN, range = !r.overflow && (errw & DERR_CELL_RANGE);
+  for (int s = 0; (scan || range) && s < nsets; s++) drop_build(*sets[s]);
+  if (scan) return {ERR_INTERNAL, r.overflow, "cell-list build: a scan tile gave up waiting for an earlier tile"};
+  if (range)
+    return {ERR_INTERNAL, false, "cell-list build consistency check failed (particle outside the computing box)"};
+  return r;
 }
 
 }  // namespace clm

@@ -14,12 +14,6 @@
 
 namespace clm {
 
-enum Status {
-  RERUN_BUILD = -1,  // internal: the copies overflowed the capacity; rebuild with the exact size and rerun
-  OK = 0, ERR_ARG = 1, ERR_CELL_TOO_SMALL = 2, ERR_NAN = 3, ERR_DIM = 4, ERR_CUDA = 5, ERR_CAPACITY = 6,
-  ERR_STATE = 7, ERR_TIMEOUT = 8, ERR_NOMEM = 9, ERR_LCELL = 10, ERR_NONPERIODIC_CELL = 11, ERR_INTERNAL = 12
-};
-
 // Process-wide count and size of the device (and pinned host) allocations the library made; steady-state
 // steps with unchanged sizes make none (reported by clm_device_allocations).
 inline std::atomic<long long>& alloc_count() {
@@ -60,7 +54,7 @@ struct DevBuf {
   template <class U> U* as() const { return static_cast<U*>(p); }
 };
 
-// One particle set and its cell list on the device.
+// One particle set and its cell list on the device (its state from build to build: BuildState).
 struct SetData : BuildState {
   int64_t n = 0;
   DevBuf x;                 // positions as given (n x dim, column-major dim x n)
@@ -69,7 +63,6 @@ struct SetData : BuildState {
   DevBuf ncopy, copy_off;   // copies per particle and their exclusive scan
   DevBuf keys[2], vals[2];  // (cell, particle<<5 | image) pairs: particle order, then grouped by cell
   DevBuf cell_count;        // one system: scan words and per-cell {copies, real} counters (zeroed per build)
-  size_t cell_count_zero = 0;  // bytes of cell_count left cleared by the last build (0: clear before use)
   DevBuf cell_start, cell_flags;
   DevBuf real_list, real_scan;
   DevBuf px, py, pz;        // copies in cell order (SoA), handle dtype
@@ -78,23 +71,8 @@ struct SetData : BuildState {
   DevBuf code;              // particle index (>= 0 real copy, -(index+1) image)
   DevBuf rs_hist;
   DevBuf minmax;            // non-periodic limits scratch
-  int64_t n_copies = 0;      // valid once the build was synchronized (pending == false)
-  int64_t n_real_cells = 0;
-  int64_t copy_cap = 0;      // capacity for copies learned from previous builds
-  int64_t cap_used = 0;      // capacity used by the last build
-  bool counted = false;      // the last build was the counting build (its largest cell is read back)
-  bool prefer_radix = false; // a counting build met a cell of more than kRadixAbovePerCell copies
-  int tile_mult = 0;         // counting build: staging slots per particle of a tile (0: from the estimate)
-  int64_t n_cells_with_particles = 0;
   int64_t ncells = 0;
-  // build of a few particles in one launch (k_build_small)
-  DevBuf small_buf;          // two sets of per-cell counters, the grid barrier, each cell's copies in arrival order
-  bool small = false;        // the last build was one
-  bool small_off = false;    // one met a cell with more copies than a bucket holds
-  // larger sets and batches: a bucket per cell (k_wrap_place)
-  int bucket_used = 0;       // places per cell of the last build (0: another build)
-  int bucket = 0;            // places that an earlier build's largest cell called for
-  bool bucket_off = false;   // one met a cell with more copies than a bucket may hold
+  DevBuf small_buf;         // k_build_small: two halves of counters, the grid barrier, each cell's copies in arrival order
 };
 
 struct ScanTemp {

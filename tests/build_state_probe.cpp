@@ -32,3 +32,33 @@ extern "C" int small_counters_probe(const int* script, int n) {
   }
   return -1;
 }
+
+// check_builds on two sets built together (kind: 0 counting, 1 one-launch, 2 bucket), with the given words of the
+// device: out = {status, overflow, then for each set dirty, pending, counters to be cleared}.
+extern "C" void check_probe(int kind, int errw, int copies, int largest, int* out) {
+  clm::BuildState S[2];
+  int words[64] = {};
+  words[40] = errw;
+  for (int s = 0; s < 2; s++) {
+    S[s].built = S[s].counted = S[s].pending = true;
+    S[s].dirty = false;
+    S[s].small = kind == 1;
+    S[s].bucket_used = kind == 2 ? 24 : 0;
+    S[s].tile_mult = 2;
+    S[s].cap_used = S[s].copy_cap = 1000;
+    S[s].small_cells = 100;
+    S[s].cell_count_zero = 800;
+    words[32 + 2 * s] = copies;
+    words[33 + 2 * s] = 10;
+    words[44 + s] = largest;
+  }
+  clm::BuildState* sets[2] = {&S[0], &S[1]};
+  const clm::BuildCheck c = clm::check_builds(sets, 2, words);
+  out[0] = c.status;
+  out[1] = c.overflow;
+  for (int s = 0; s < 2; s++) {
+    out[2 + 3 * s] = S[s].dirty;
+    out[3 + 3 * s] = S[s].pending;
+    out[4 + 3 * s] = S[s].small_cells == 0 && S[s].cell_count_zero == 0;
+  }
+}
