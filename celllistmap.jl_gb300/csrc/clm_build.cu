@@ -4,8 +4,7 @@
 // of add_particles! 940-950 and add_particle_to_celllist! 983-1057) and the
 // non-periodic build (src/internals/NonPeriodicCells.jl:93-251).
 //
-// One system of at most 2^16 particles: k_build_small, the whole build in one cooperative launch (both sets of an x-y
-// handle together).
+// One system of at most 2^16 particles: k_small_place and k_small_cells (both sets of an x-y handle together).
 // Larger systems and batches (bucket build, three launches):
 //   k_wrap_place    wrap into the first cell (wrap_to_first, CellOperations.jl:91-94),
 //                   rotate, test the 3^N-1 translation images against the computing
@@ -815,21 +814,22 @@ __global__ void __launch_bounds__(kBlock) k_bucket_gather(const __grid_constant_
   }
 }
 
-// ------------------------------------------------------------------ one system of few particles: one launch
-// The whole build in one cooperative kernel, for sets of at most kSmallParticles: the four kernels of the
-// counting build are each a few us of latency at these sizes.  Every warp wraps its particles (warps of
+// ------------------------------------------------------------------ one system of few particles: two launches
+// The build of sets of at most kSmallParticles, both sets of an x-y handle together: the three or four kernels of the
+// other builds are each a few us of latency at these sizes.  k_small_place: every warp wraps its particles (warps of
 // different blocks take neighbouring chunks, so that a thousand particles occupy 32 SMs and not four: a
 // warp's FP64 instruction holds its SM's pipe for 16 cycles), and every copy takes a slot of its cell's bucket
-// with one atomic.  After a barrier over the grid each block takes a range of cells: it sums the counts of the
+// with one atomic.  k_small_cells: each block takes a range of cells: it sums the counts of the
 // cells before it, writes their starts and the real-cell list, and its warps rank the copies of a cell by
 // value (particle-index order) and gather them.  A cell with more than kBucket copies is flagged
 // (DERR_TILE_OVERFLOW) and the set is built by the other kernels from then on.
+// Not one cooperative launch with a barrier over its grid: that waits until the device has room for all of its blocks at
+// once, and never starts beside a kernel that holds most of the multiprocessors until this step is done.  It built 1 to
+// 2 us faster (32,000 particles 22 / 27 us); the steps of 1,003 and 32,000 particles took the same time (82 and 76 us).
 constexpr int kSmallThreads = 512;
 constexpr int kBucket = 128;
-// Up to here the one launch is clearly the shorter build (GB300, Float32 / Float64 at liquid density, against the
-// bucket build: 4,000 particles 18 / 21 us against 28 / 33, 32,000 22 / 27 against 30 / 35, 64,000 26 / 36 against
-// 31 / 41).  At 96,000 they are even (32 / 43 against 33 / 44), and its blocks wait for a whole free device; at 400,000
-// it is the longer one (68 / 108 against 47 / 77).
+// Up to here this is the shorter build (GB300, Float32 / Float64 at liquid density: 4,000 particles 19 / 22 us against
+// 28 / 33 of the bucket build, 32,000 23 / 28 against 30 / 35, 65,536 28 / 36 against 32 / 39 for one particle more).
 constexpr int64_t kSmallParticles = 1 << 16;
 constexpr int64_t kSmallCells = 1 << 15;
 constexpr double kSmallPerCell = 64.0;  // copies per cell expected at uniform density: half a bucket
@@ -837,9 +837,7 @@ constexpr double kSmallPerCell = 64.0;  // copies per cell expected at uniform d
 template <class T> struct SmallSet {
   PlaceArgs<T> P;
   int ncells, cap;
-  int* cf_next;       // the next build's counters, cleared here
-  unsigned* bar;      // {arrived, generation}
-  unsigned epoch;     // this launch's generation
+  int* cf_next;       // the next build's counters, cleared by k_small_place
   int* cell_start;
   int* cell_flags;
   int* real_list;
@@ -853,55 +851,43 @@ template <class T> struct SmallSet {
   int* code;
 };
 
-// Both sets of an x-y handle in one launch: blocks [0, split) build set 0, the others set 1, each group with its own
-// barrier.
+// Both sets of an x-y handle in one launch: blocks [0, split) build set 0, the others set 1.
 template <class T> struct SmallBuild {
   DevGeom<T> g;
   SmallSet<T> set[2];
   int split;
 };
+// This block's set, its number among the set's blocks and their number.
+template <class T> __device__ __forceinline__ const SmallSet<T>& small_set(const SmallBuild<T>& A, int& block, int& blocks) {
+  const bool second = (int)blockIdx.x >= A.split;
+  block = (int)blockIdx.x - (second ? A.split : 0);
+  blocks = second ? (int)gridDim.x - A.split : A.split;
+  return A.set[second ? 1 : 0];
+}
 
 template <class T, int N, int SH>
-__global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_constant__ SmallBuild<T> A) {
-  const DevGeom<T>& g = A.g;
-  const bool second = (int)blockIdx.x >= A.split;
-  const SmallSet<T>& B = A.set[second ? 1 : 0];
-  const int block = (int)blockIdx.x - (second ? A.split : 0), blocks = second ? (int)gridDim.x - A.split : A.split;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int kW = kSmallThreads / 32;
+__global__ void __launch_bounds__(kSmallThreads) k_small_place(const __grid_constant__ SmallBuild<T> A) {
+  int block, blocks;
+  const SmallSet<T>& B = small_set(A, block, blocks);
   __shared__ PlaceShared<T, N, kSmallThreads> sm;
-  load_shift<T>(g, sm.shift);
+  load_shift<T>(A.g, sm.shift);
+  if (block == 0 && threadIdx.x == 0) *B.max_cell = 0;
   for (int c = block * kSmallThreads + threadIdx.x; c < 2 * B.ncells; c += blocks * kSmallThreads) B.cf_next[c] = 0;
-  for (int i0 = block * 32; i0 < B.P.n; i0 += kW * blocks * 32) {
-    place_copies<T, N, SH, kSmallThreads, false>(g, B.P, i0, blocks * 32, sm);
+  for (int i0 = block * 32; i0 < B.P.n; i0 += kSmallThreads * blocks) {
+    place_copies<T, N, SH, kSmallThreads, false>(A.g, B.P, i0, blocks * 32, sm);
     __syncthreads();
   }
-  // ---- barrier over the set's blocks (all are resident: cooperative launch).  The last block to arrive opens it.
-  __shared__ int s_ok;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s_ok = 1;
-    if (atomicAdd(&B.bar[0], 1u) == (unsigned)blocks - 1u) {
-      B.bar[0] = 0u;
-      __threadfence();
-      atomicExch(&B.bar[1], B.epoch);
-    } else {
-      int spins = 0;
-      while (*(volatile unsigned*)&B.bar[1] != B.epoch) {
-        if (++spins > kScanSpinLimit) {
-          atomicOr(B.P.err, DERR_SCAN);
-          s_ok = 0;
-          break;
-        }
-        __nanosleep(20);
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  if (!s_ok) return;
-  // ---- this block's cells; what other blocks wrote is read past L1 (__ldcg)
+}
+
+template <class T, int N>
+__global__ void __launch_bounds__(kSmallThreads) k_small_cells(const __grid_constant__ SmallBuild<T> A) {
+  const DevGeom<T>& g = A.g;
+  int block, blocks;
+  const SmallSet<T>& B = small_set(A, block, blocks);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kW = kSmallThreads / 32;
+  __shared__ T s_shift[27][3];
+  load_shift<T>(g, s_shift);
   const int per = (B.ncells + blocks - 1) / blocks;
   const int c0 = min(B.ncells, block * per), c1 = min(B.ncells, c0 + per);
   __shared__ int s_sum[2][kW];
@@ -947,8 +933,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_cons
       if (c == B.ncells - 1) {
         B.cell_start[B.ncells] = start + v.x;
         *B.n_real = fpos + v.y;
-        *B.max_cell = 0;
       }
+      if (v.x > kBucket) atomicMax(B.max_cell, v.x);
       if (start + v.x > B.cap) atomicOr(B.P.err, DERR_COPY_OVERFLOW);
     }
     __syncthreads();
@@ -991,7 +977,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_build_small(const __grid_cons
         T w[N];
 #pragma unroll
         for (int d = 0; d < N; d++) w[d] = __ldcg(&B.P.wrapped[(int64_t)p * N + d]);
-        gather_copy<T, N>(g, sm.shift, w, s + r[q], p, k, c, B.px, B.py, B.pz, B.off, B.xq, B.code);
+        gather_copy<T, N>(g, s_shift, w, s + r[q], p, k, c, B.px, B.py, B.pz, B.off, B.xq, B.code);
       }
     }
   }
@@ -1104,7 +1090,7 @@ __global__ void k_compact(const int* __restrict__ flags, const int* __restrict__
 // Limits of both sets in one launch: a block reduces its share of a set (blockIdx.y) to partials, and the last block
 // of each set to finish reduces those and writes {lo, hi} to the host's pinned words.  The host needs the limits
 // before it can lay out the cells, so this is latency only: one launch and one wait, not a launch, a copy through
-// pageable memory and a wait per set (with the one launch of k_build_small for both sets, the build of 1501 and 4507
+// pageable memory and a wait per set (with joint launches of the build for both sets, the build of 1501 and 4507
 // points went from 82 to 42 us).
 constexpr int kLimitBlocks = 256;
 template <class T> struct LimitArgs {
@@ -1290,11 +1276,11 @@ template <class T> int64_t copy_capacity(const SetData& S, const Geometry<T>& g)
   return std::max<int64_t>(std::max<int64_t>(S.copy_cap, (int64_t)est), n + 64);
 }
 
-// One system of few particles, for k_build_small: the set's buffers and its part of the launch.
+// One system of few particles, for k_small_place and k_small_cells: the set's buffers and its part of the launches.
 template <class T>
 int prepare_small(Handle& h, SetData& S, int N, int64_t n, int64_t ncells, int64_t cap, SmallSet<T>& B) {
-  // the counters of this build and the next, the barrier, and the buckets
-  const size_t words = 4 * (size_t)ncells + 2;
+  // the counters of this build and the next, and the buckets
+  const size_t words = 4 * (size_t)ncells;
   const void* at = S.small_buf.p;
   if (!S.small_buf.reserve(sizeof(int) * (words + kBucket * (size_t)ncells)) ||
       !S.wrapped.reserve(sizeof(T) * N * n) || !S.px.reserve(sizeof(T) * cap) || !S.py.reserve(sizeof(T) * cap) ||
@@ -1316,8 +1302,6 @@ int prepare_small(Handle& h, SetData& S, int N, int64_t n, int64_t ncells, int64
   B.ncells = (int)ncells;
   B.cap = (int)cap;
   B.cf_next = S.small_buf.as<int>() + 2 * ncells * (1 - half);
-  B.bar = reinterpret_cast<unsigned*>(S.small_buf.as<int>() + 4 * ncells);
-  B.epoch = S.small_epoch + 1;
   B.cell_start = S.cell_start.as<int>();
   B.cell_flags = S.cell_flags.as<int>();
   B.real_list = S.real_list.as<int>();
@@ -1332,45 +1316,42 @@ int prepare_small(Handle& h, SetData& S, int N, int64_t n, int64_t ncells, int64
   return OK;
 }
 
-// Blocks of the one-launch build (one per SM); 0 if the device has no cooperative launch.
+// Blocks of the build of few particles: one per SM.
 inline int small_blocks() {
   static const int sms = [] {
-    int v = 0, dev = 0, coop = 0;
+    int v = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    return coop && v >= 2 ? v : 0;
+    return std::max(2, v);
   }();
   return sms;
 }
 
-// The launch for the sets that were prepared (`which`; `count` of them, in A.set[0] and then A.set[1]).
-// `refused`: the device cannot hold the grid at once (a part of it only, for this process).
-template <class T> int launch_small(Handle& h, SmallBuild<T>& A, unsigned which, int count, int N, bool* refused) {
+// The launches for the sets that were prepared (`which`; `count` of them, in A.set[0] and then A.set[1]).
+template <class T> int launch_small(Handle& h, SmallBuild<T>& A, unsigned which, int count, int N) {
   using Kernel = void (*)(const SmallBuild<T>);
-  Kernel k = (N == 3) ? (Kernel)k_build_small<T, 3, kShapeGeneral> : (Kernel)k_build_small<T, 2, kShapeGeneral>;
+  Kernel place = (N == 3) ? (Kernel)k_small_place<T, 3, kShapeGeneral> : (Kernel)k_small_place<T, 2, kShapeGeneral>;
   if constexpr (std::is_same<T, double>::value) {
-    if (N == 3 && A.g.shape == kShapeDiag) k = k_build_small<T, 3, kShapeDiag>;
-    else if (N == 3 && A.g.shape == kShapeUpper) k = k_build_small<T, 3, kShapeUpper>;
+    if (N == 3 && A.g.shape == kShapeDiag) place = k_small_place<T, 3, kShapeDiag>;
+    else if (N == 3 && A.g.shape == kShapeUpper) place = k_small_place<T, 3, kShapeUpper>;
   }
+  const Kernel cells = (N == 3) ? (Kernel)k_small_cells<T, 3> : (Kernel)k_small_cells<T, 2>;
   const int blocks = small_blocks();
   A.split = blocks;
   if (count == 2) {  // blocks in proportion to the particles, and at least an eighth each
     const double share = (double)A.set[0].P.n / ((double)A.set[0].P.n + (double)A.set[1].P.n);
     A.split = std::min(std::max((int)(share * blocks), std::max(1, blocks / 8)), blocks - std::max(1, blocks / 8));
   }
-  void* args[] = {&A};
-  const cudaError_t e =
-      cudaLaunchCooperativeKernel((const void*)k, dim3((unsigned)blocks), dim3(kSmallThreads), args, 0, h.stream);
-  *refused = e == cudaErrorCooperativeLaunchTooLarge;
+  place<<<(unsigned)blocks, kSmallThreads, 0, h.stream>>>(A);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) {
+    cells<<<(unsigned)blocks, kSmallThreads, 0, h.stream>>>(A);
+    e = cudaGetLastError();
+  }
   for (int s = 0; s < h.nsets; s++)
     if (which >> s & 1u) small_launched(h.sets[s], h.sets[s].ncells, e == cudaSuccess);
-  if (*refused) {
-    cudaGetLastError();
-    return OK;
-  }
   CLM_CUDA_TRY(h, e);
-  h.launches++;
+  h.launches += 2;
   return OK;
 }
 
@@ -1551,7 +1532,7 @@ int build_bucket(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, 
   return OK;
 }
 
-// `small`: where a set that k_build_small takes leaves its part of the launch (`count` sets so far).
+// `small`: where a set of few particles leaves its part of the joint launches (`count` sets so far).
 template <class T> int build_set(Handle& h, int set, const Geometry<T>& g, SmallBuild<T>& small, int& count) {
   SetData& S = h.sets[set];
   const int N = g.dim;
@@ -1610,7 +1591,7 @@ template <class T> int build_set(Handle& h, int set, const Geometry<T>& g, Small
   S.counted = !batch && !crowded;
   S.small = false;
   S.bucket_used = 0;
-  if (!batch && small_blocks() > 0 && !S.prefer_radix && !S.small_off && n <= kSmallParticles && ncells <= kSmallCells &&
+  if (!batch && !S.prefer_radix && !S.small_off && n <= kSmallParticles && ncells <= kSmallCells &&
       copies_expected(S, g) <= kSmallPerCell * (double)ncells) {
     small.g = dg;
     const int st = prepare_small<T>(h, S, N, n, ncells, cap, small.set[count]);
@@ -1769,26 +1750,16 @@ template <class T> int build_set(Handle& h, int set, const Geometry<T>& g, Small
 
 // Builds the sets of `which` (bit s: set s), all enqueued on the handle's stream.
 template <class T> int enqueue_builds(Handle& h, const Geometry<T>& g, unsigned which) {
-  for (bool again = true; again;) {
-    SmallBuild<T> small;
-    int count = 0;
-    unsigned in_small = 0;
-    for (int s = 0; s < h.nsets; s++) {
-      if (!(which >> s & 1u)) continue;
-      const int before = count, st = build_set<T>(h, s, g, small, count);
-      if (st) return st;
-      if (count > before) in_small |= 1u << s;
-    }
-    again = false;
-    if (count) {
-      const int st = launch_small<T>(h, small, in_small, count, g.dim, &again);
-      if (st) return st;
-    }
-    which = again ? in_small : 0;  // refused: those sets again, by the other builds
-    for (int s = 0; s < h.nsets; s++)
-      if (which >> s & 1u) h.sets[s].small_off = true;
+  SmallBuild<T> small;
+  int count = 0;
+  unsigned in_small = 0;
+  for (int s = 0; s < h.nsets; s++) {
+    if (!(which >> s & 1u)) continue;
+    const int before = count, st = build_set<T>(h, s, g, small, count);
+    if (st) return st;
+    if (count > before) in_small |= 1u << s;
   }
-  return OK;
+  return count ? launch_small<T>(h, small, in_small, count, g.dim) : OK;
 }
 // When one fails, none of them counts as built: a set that was only prepared for the joint launch was not.
 template <class T> int build_sets(Handle& h, const Geometry<T>& g, unsigned which) {

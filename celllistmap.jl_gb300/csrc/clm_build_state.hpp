@@ -33,17 +33,17 @@ struct BuildState {
   bool prefer_radix = false; // one met a cell of more than kRadixAbovePerCell copies
   int tile_mult = 0;         // counting build: staging slots per particle of a tile (0: from the estimate)
   size_t cell_count_zero = 0;  // bytes of the scan words and counters left cleared by the last build (0: clear before use)
-  bool small = false;        // the last build was k_build_small
+  bool small = false;        // the last build was that of few particles (k_small_place)
   bool small_off = false;    // one met a cell with more copies than a bucket holds
   int bucket_used = 0;       // bucket build: places per cell of the last build (0: another build)
   int bucket = 0;            // places that an earlier build's largest cell called for
   bool bucket_off = false;   // one met a cell with more copies than a bucket may hold
-  // k_build_small: two halves of per-cell counters.  A launch counts in one half and clears the other for the next.
+  // k_small_place: two halves of per-cell counters.  A launch counts in one half and clears the other for the next.
   int64_t small_cells = 0;   // cells that they are laid out and cleared for (0: none)
   unsigned small_epoch = 0;  // launches since they were cleared
 };
 
-// Before a launch of k_build_small that counts `ncells` cells (`moved`: in a new allocation): true when both halves have
+// Before a launch of k_small_place that counts `ncells` cells (`moved`: in a new allocation): true when both halves have
 // to be cleared first.
 inline bool small_needs_clear(BuildState& S, int64_t ncells, bool moved) {
   if (S.small_cells == ncells && !moved) return false;

@@ -72,7 +72,7 @@ struct SetData : BuildState {
   DevBuf rs_hist;
   DevBuf minmax;            // non-periodic limits scratch
   int64_t ncells = 0;
-  DevBuf small_buf;         // k_build_small: two halves of counters, the grid barrier, each cell's copies in arrival order
+  DevBuf small_buf;         // few particles: two halves of counters, each cell's copies in arrival order
 };
 
 struct ScanTemp {

@@ -5,7 +5,7 @@
 
 #include "clm_build_state.hpp"
 
-// Builds of one set with k_build_small's counters: step k of `script` is 0 (prepared and launched), 1 (prepared, dropped
+// Builds of one set with the counters of k_small_place: step k of `script` is 0 (prepared and launched), 1 (prepared, dropped
 // because the other set failed), 2 (prepared, the launch failed), 3 (launched with another number of cells) or 4
 // (launched in a new allocation).  Returns the first step whose launch found counters that were not clear, or -1.
 extern "C" int small_counters_probe(const int* script, int n) {
@@ -33,7 +33,7 @@ extern "C" int small_counters_probe(const int* script, int n) {
   return -1;
 }
 
-// check_builds on two sets built together (kind: 0 counting, 1 one-launch, 2 bucket), with the given words of the
+// check_builds on two sets built together (kind: 0 counting, 1 few particles, 2 bucket), with the given words of the
 // device: out = {status, overflow, then for each set dirty, pending, counters to be cleared}.
 extern "C" void check_probe(int kind, int errw, int copies, int largest, int* out) {
   clm::BuildState S[2];

@@ -1,5 +1,5 @@
 """What a particle set remembers from one build to the next (clm_build_state.hpp): the alternating counters of the
-one-launch build start clear after every mixture of launches, dropped and failed ones, and a list that a build with an
+small build start clear after every mixture of launches, dropped and failed ones, and a list that a build with an
 error left is never used by a later call.  Runs on the CPU."""
 import ctypes as C
 import itertools

@@ -1,4 +1,4 @@
-"""A small set with a NaN coordinate: its build (k_build_small) leaves a whole cell list of the other particles, because
+"""A small set with a NaN coordinate: its build (k_small_place, k_small_cells) leaves a whole cell list of the other particles, because
 the map enqueued behind it runs before the host reads the error.  The call answers with the NaN error, and the steps
 after it, on this handle and on another one, equal the oracle."""
 import ctypes as C
