@@ -561,6 +561,7 @@ int32_t clm_batched_set_systems(clm_handle h, int64_t nsys, const int64_t* offse
   B.offsets.swap(off);
   B.cells.swap(cm);
   B.tables_ready = false;
+  forget_crowding(h->sets[0]);
   B.status.assign((size_t)nsys, OK);
   h->kind = cell_kind;
   h->lcell = lcell;

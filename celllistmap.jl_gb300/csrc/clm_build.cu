@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(WE_BLOCK) k_wrap_emit(DevGeom<T> g, const T* _
 // WE_BLOCK particles in the tile's own range of `slots` staging slots (the in-cell ranking orders a cell by
 // value, so the copies need no position in particle order, and no tile waits on an earlier one).  Each
 // tile writes its number of copies; a tile with more copies than slots writes none and flags
-// DERR_TILE_OVERFLOW (the build is repeated with more slots).  Every copy adds one to its cell's counter
+// `over` (tile_overflow; the build is repeated with more slots).  Every copy adds one to its cell's counter
 // (the lanes of a warp whose copies share a cell with one add) and the real copy marks its cell; cell_cf
 // holds {copies, holds a real particle} per cell, zeroed before the launch.  Tile 0 clears the word of
 // the largest cell that k_cell_scan finds.
@@ -418,7 +418,7 @@ template <class T, int N, int SH = kShapeGeneral>
 __global__ void __launch_bounds__(WE_BLOCK) k_wrap_stage(DevGeom<T> g, const T* __restrict__ x, int n,
                                                        T* __restrict__ wrapped, int slots, uint32_t* __restrict__ keys,
                                                        uint32_t* __restrict__ vals, int* __restrict__ tile_count,
-                                                       int* __restrict__ cell_cf, int* __restrict__ max_cell,
+                                                       int* __restrict__ cell_cf, int* __restrict__ max_cell, int over,
                                                        int* __restrict__ err) {
   static_assert(WE_PPT == 1, "one particle per thread");
   __shared__ int wsum[WE_BLOCK / 32 + 1];
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(WE_BLOCK) k_wrap_stage(DevGeom<T> g, const T* 
   if (agg > slots) nc = 0;  // the whole tile (agg is the tile's)
   if (threadIdx.x == 0) {
     tile_count[tile] = (agg > slots) ? 0 : agg;
-    if (agg > slots) atomicOr(err, DERR_TILE_OVERFLOW);
+    if (agg > slots) atomicOr(err, over);
   }
   const int64_t base = (int64_t)tile * slots + v[0] + off;
   // the copies of the particle (the real copy, then the images in increasing image code), walked by the
@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(kBlock) k_rank_gather(DevGeom<T> g, const T* _
 // ------------------------------------------------------------------ buckets: wrap and place, gather
 // The builds that place every copy once: each cell has `slots` places, and a copy takes the next one of its cell with
 // one atomic when its key is known, so no list of keys is written, read back and scattered.  A cell with more copies
-// than places sets DERR_TILE_OVERFLOW (the build is repeated with more places, or by the counting build).
+// than places sets the set's tile_overflow bit (the build is repeated with more places, or by the counting build).
 //
 // A warp's copies are shared out evenly over its block before their cells are computed: most particles have one
 // copy, a few have seven, and lanes that walked their own would leave the others idle (and in Float64 hold the FP64
@@ -640,6 +640,7 @@ template <class T> struct PlaceArgs {
   int slots;
   int* cf;           // {copies, holds a real particle} per cell, zero before the build
   int* err;
+  int over;          // the set's bit for a cell with more copies than places
 };
 template <class T, int N, int NT> struct PlaceShared {
   T pos[NT][N];
@@ -716,7 +717,7 @@ __device__ __forceinline__ void place_copies(const DevGeom<T>& G, const PlaceArg
     if (real) P.cf[2 * (int64_t)key + 1] = 1;
     const int at = first + (t >> 5) * stride + (t & 31);
     if (slot < P.slots) P.bucket[(int64_t)key * P.slots + slot] = ((uint32_t)at << 5) | (uint32_t)k;
-    else atomicOr(P.err, DERR_TILE_OVERFLOW);
+    else atomicOr(P.err, P.over);
   }
 }
 
@@ -754,7 +755,7 @@ __global__ void __launch_bounds__(kBlock) k_bucket_gather(const __grid_constant_
   const int c0 = blockIdx.x * per, nc = min(per, ncells - c0);
   for (int t = threadIdx.x; t <= nc; t += kBlock) s_start[t] = cell_start[c0 + t];
   if (!BATCH) load_shift<T>(G, s_shift);
-  if (*(volatile int*)P.err & DERR_TILE_OVERFLOW) return;  // set by k_wrap_place: the list is not used
+  if (*(volatile int*)P.err & P.over) return;  // set by k_wrap_place: the list is not used
   __syncthreads();
   const int base = s_start[0], tot = s_start[nc] - base;
   if (tot < 0 || tot > per * P.slots || base < 0) {  // the same in every thread
@@ -822,12 +823,11 @@ __global__ void __launch_bounds__(kBlock) k_bucket_gather(const __grid_constant_
 // with one atomic.  k_small_cells: each block takes a range of cells: it sums the counts of the
 // cells before it, writes their starts and the real-cell list, and its warps rank the copies of a cell by
 // value (particle-index order) and gather them.  A cell with more than kBucket copies is flagged
-// (DERR_TILE_OVERFLOW) and the set is built by the other kernels from then on.
+// (tile_overflow) and the set is built by the other kernels until its cells are emptier again (check_builds).
 // Not one cooperative launch with a barrier over its grid: that waits until the device has room for all of its blocks at
 // once, and never starts beside a kernel that holds most of the multiprocessors until this step is done.  It built 1 to
 // 2 us faster (32,000 particles 22 / 27 us); the steps of 1,003 and 32,000 particles took the same time (82 and 76 us).
 constexpr int kSmallThreads = 512;
-constexpr int kBucket = 128;
 // Up to here this is the shorter build (GB300, Float32 / Float64 at liquid density: 4,000 particles 19 / 22 us against
 // 28 / 33 of the bucket build, 32,000 23 / 28 against 30 / 35, 65,536 28 / 36 against 32 / 39 for one particle more).
 constexpr int64_t kSmallParticles = 1 << 16;
@@ -917,7 +917,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_cells(const __grid_cons
   }
   // An overflow: nothing maps this list.  A NaN particle has no copies, and what the others have is gathered all the
   // same: the map that was enqueued behind this build runs over the list, and the other set's list stays in use.
-  const bool skip = (__ldcg(B.P.err) & DERR_TILE_OVERFLOW) != 0;
+  const bool skip = (__ldcg(B.P.err) & B.P.over) != 0;
   for (int cb = c0; cb < c1; cb += kSmallThreads) {  // 512 cells at a time
     const int c = cb + threadIdx.x;
     int2 v = make_int2(0, 0);
@@ -1299,6 +1299,7 @@ int prepare_small(Handle& h, SetData& S, int N, int64_t n, int64_t ncells, int64
   B.P.slots = kBucket;
   B.P.cf = S.small_buf.as<int>() + 2 * ncells * half;
   B.P.err = h.err.as<int>();
+  B.P.over = tile_overflow((int)(&S - h.sets));
   B.ncells = (int)ncells;
   B.cap = (int)cap;
   B.cf_next = S.small_buf.as<int>() + 2 * ncells * (1 - half);
@@ -1391,6 +1392,7 @@ int build_counting(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n
   if (S.cell_count_zero < zero_bytes) CLM_CUDA_TRY(h, cudaMemsetAsync(z, 0, zero_bytes, h.stream));
   S.cell_count_zero = 0;
   int* tile_count = S.ncopy.as<int>();
+  const int over = tile_overflow((int)(&S - h.sets));
   int* max_cell = S.copy_off.as<int>() + n + 1;  // the largest cell
   // Float64 3D cells whose input matrix has exact zeros take a wrap that skips them (wrap_point_shaped)
   bool shaped = false;
@@ -1398,23 +1400,23 @@ int build_counting(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n
     if (N == 3 && dg.shape == kShapeDiag) {
       k_wrap_stage<T, 3, kShapeDiag><<<(unsigned)tiles, WE_BLOCK, 0, h.stream>>>(
           dg, S.x.as<T>(), (int)n, S.wrapped.as<T>(), slots, S.keys[0].as<uint32_t>(), S.vals[0].as<uint32_t>(),
-          tile_count, cell_cf, max_cell, err);
+          tile_count, cell_cf, max_cell, over, err);
       shaped = true;
     } else if (N == 3 && dg.shape == kShapeUpper) {
       k_wrap_stage<T, 3, kShapeUpper><<<(unsigned)tiles, WE_BLOCK, 0, h.stream>>>(
           dg, S.x.as<T>(), (int)n, S.wrapped.as<T>(), slots, S.keys[0].as<uint32_t>(), S.vals[0].as<uint32_t>(),
-          tile_count, cell_cf, max_cell, err);
+          tile_count, cell_cf, max_cell, over, err);
       shaped = true;
     }
   }
   if (!shaped && N == 3)
     k_wrap_stage<T, 3><<<(unsigned)tiles, WE_BLOCK, 0, h.stream>>>(dg, S.x.as<T>(), (int)n, S.wrapped.as<T>(), slots,
                                                                   S.keys[0].as<uint32_t>(), S.vals[0].as<uint32_t>(),
-                                                                  tile_count, cell_cf, max_cell, err);
+                                                                  tile_count, cell_cf, max_cell, over, err);
   else if (!shaped)
     k_wrap_stage<T, 2><<<(unsigned)tiles, WE_BLOCK, 0, h.stream>>>(dg, S.x.as<T>(), (int)n, S.wrapped.as<T>(), slots,
                                                                   S.keys[0].as<uint32_t>(), S.vals[0].as<uint32_t>(),
-                                                                  tile_count, cell_cf, max_cell, err);
+                                                                  tile_count, cell_cf, max_cell, over, err);
   CLM_CUDA_TRY(h, cudaGetLastError());
   h.launches++;
   k_cell_scan<<<(unsigned)ct, kBlock, 0, h.stream>>>(cell_cf, (int)ncells, S.cell_start.as<int>(), S.cell_flags.as<int>(),
@@ -1496,6 +1498,7 @@ int build_bucket(Handle& h, SetData& S, const DevGeom<T>& dg, int N, int64_t n, 
   P.slots = slots;
   P.cf = cell_cf;
   P.err = err;
+  P.over = tile_overflow((int)(&S - h.sets));
   using Place = void (*)(const DevGeom<T>, const PlaceArgs<T>, int*);
   Place place;
   if (batch) place = (N == 3) ? (Place)k_wrap_place<T, 3, kShapeGeneral, true> : (Place)k_wrap_place<T, 2, kShapeGeneral, true>;
@@ -1555,6 +1558,8 @@ template <class T> int build_set(Handle& h, int set, const Geometry<T>& g, Small
       !S.real_scan.reserve(sizeof(int) * (ncells + 1)) || !S.real_list.reserve(sizeof(int) * (ncells + 1)) ||
       !S.copy_off.reserve(sizeof(int) * (n + 2)))  // copies per particle scan, total, largest cell
     return ERR_NOMEM;
+  S.small = false;
+  S.bucket_used = 0;
   if (n == 0) CLM_CUDA_TRY(h, cudaMemsetAsync(S.cell_flags.p, 0, sizeof(int) * (ncells + 1), h.stream));
   S.built = true;
   S.dirty = false;
@@ -1589,8 +1594,6 @@ template <class T> int build_set(Handle& h, int set, const Geometry<T>& g, Small
   // sort's cost does not depend on it.  Either gives the same cell list.
   const bool crowded = !batch && (S.prefer_radix || (double)cap > kCountingMaxPerCell * (double)ncells);
   S.counted = !batch && !crowded;
-  S.small = false;
-  S.bucket_used = 0;
   if (!batch && !S.prefer_radix && !S.small_off && n <= kSmallParticles && ncells <= kSmallCells &&
       copies_expected(S, g) <= kSmallPerCell * (double)ncells) {
     small.g = dg;

@@ -18,7 +18,8 @@ enum Status {
 
 // Cells of more copies than this are built by radix (the counting build ranks each copy against its cell).
 constexpr int kRadixAbovePerCell = 1024;
-// The most places per cell that the bucket build takes.
+// Places per cell of the build of few particles, and the most that the bucket build takes.
+constexpr int kBucket = 128;
 constexpr int kBucketMost = 256;
 
 struct BuildState {
@@ -34,10 +35,10 @@ struct BuildState {
   int tile_mult = 0;         // counting build: staging slots per particle of a tile (0: from the estimate)
   size_t cell_count_zero = 0;  // bytes of the scan words and counters left cleared by the last build (0: clear before use)
   bool small = false;        // the last build was that of few particles (k_small_place)
-  bool small_off = false;    // one met a cell with more copies than a bucket holds
+  bool small_off = false;    // one met a cell with more copies than kBucket
   int bucket_used = 0;       // bucket build: places per cell of the last build (0: another build)
   int bucket = 0;            // places that an earlier build's largest cell called for
-  bool bucket_off = false;   // one met a cell with more copies than a bucket may hold
+  bool bucket_off = false;   // a build met a cell with more copies than kBucketMost leaves room for
   // k_small_place: two halves of per-cell counters.  A launch counts in one half and clears the other for the next.
   int64_t small_cells = 0;   // cells that they are laid out and cleared for (0: none)
   unsigned small_epoch = 0;  // launches since they were cleared
@@ -64,6 +65,15 @@ inline void small_launched(BuildState& S, int64_t ncells, bool ok) {
 inline void drop_build(BuildState& S) {
   S.pending = false;
   S.dirty = true;
+}
+
+// Places per cell for cells of up to `most` copies, a quarter more.
+inline int bucket_places(int most) { return (most + most / 4 + 7) / 8 * 8; }
+
+// A set (or a batch) whose fullest cells are no longer those of earlier builds.
+inline void forget_crowding(BuildState& S) {
+  S.small_off = S.bucket_off = S.prefer_radix = false;
+  S.bucket = 0;
 }
 
 struct BuildCheck {
@@ -98,26 +108,30 @@ inline BuildCheck check_builds(BuildState* const* sets, int nsets, const int* wo
     }
     S.n_copies = words[32 + 2 * s];
     S.n_real_cells = words[33 + 2 * s];
-    if (S.counted && words[44 + s] > kRadixAbovePerCell) S.prefer_radix = true;
-    if (S.small && (errw & DERR_TILE_OVERFLOW)) {
-      // a cell had more copies than its bucket: the counting build (or radix, when it finds the cell crowded)
-      S.small_off = S.bucket_off = true;
-      S.dirty = true;
-      r.overflow = true;
-    } else if (S.bucket_used && (errw & DERR_TILE_OVERFLOW)) {
-      // more places than the largest cell's copies, or the other builds
-      const int most = words[44 + s], want = (most + most / 4 + 7) / 8 * 8;
-      if (most > S.bucket_used) {
-        if (want <= kBucketMost) S.bucket = want;
+    // the largest cell's copies (k_small_cells: 0 when every cell fits its bucket)
+    const int most = S.counted ? words[44 + s] : 0;
+    if (most > kRadixAbovePerCell) S.prefer_radix = true;
+    if (errw & tile_overflow(s)) {
+      if (S.small || S.bucket_used) {
+        // more places than the largest cell's copies, or the builds without buckets
+        if (S.small) S.small_off = true;
+        if (bucket_places(most) <= kBucketMost) S.bucket = std::max(S.bucket, bucket_places(most));
         else S.bucket_off = true;
+      } else {
+        // a tile had more copies than its staging slots: more slots per particle, and build again
+        S.tile_mult = std::min(27, 2 * S.tile_mult);
       }
       S.dirty = true;
       r.overflow = true;
-    } else if (S.counted && (errw & DERR_TILE_OVERFLOW)) {
-      // a tile had more copies than its staging slots: more slots per particle, and build again
-      S.tile_mult = std::min(27, 2 * S.tile_mult);
-      S.dirty = true;
-      r.overflow = true;
+    } else if (S.counted && !S.small) {
+      // Cells that have become emptier: the builds given up are taken again once the fullest cell leaves a quarter of
+      // their places free, so that a set near the line does not overflow every other step.
+      if (4 * most <= 3 * kBucket) S.small_off = false;
+      if (S.bucket_off && 4 * most <= 3 * kBucketMost) {
+        S.bucket_off = false;
+        S.bucket = bucket_places(most);
+      }
+      if (2 * most <= S.bucket) S.bucket = bucket_places(most);
     }
     S.pending = false;
     if (S.n_copies > S.cap_used || (errw & DERR_COPY_OVERFLOW)) {

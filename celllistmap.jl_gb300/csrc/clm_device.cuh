@@ -605,7 +605,13 @@ enum DevError : int {
   DERR_COPY_OVERFLOW = 4,
   DERR_NL_OVERFLOW = 8,
   DERR_SCAN = 16,  // a single-pass scan gave up waiting for the prefix of an earlier tile
-  DERR_TILE_OVERFLOW = 64,  // a tile of the counting build had more copies than its staging slots
+  // a cell had more copies than its bucket, or a tile of the counting build more than its staging slots: the list is not
+  // used and the set is built again.  One bit per set (tile_overflow)
+  DERR_TILE_OVERFLOW = 64,
+  DERR_TILE_OVERFLOW_Y = 128,
 };
+__host__ __device__ constexpr int tile_overflow(int set) { return DERR_TILE_OVERFLOW << set; }
+// Builds whose list is not mapped.
+constexpr int kBuildFailed = DERR_COPY_OVERFLOW | DERR_TILE_OVERFLOW | DERR_TILE_OVERFLOW_Y | DERR_SCAN;
 
 }  // namespace clm

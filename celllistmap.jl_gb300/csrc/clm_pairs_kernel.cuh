@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
   const int gw = blockIdx.x * kWarps + warp;
   const int nw = gridDim.x * kWarps;
   // a build that flagged an overflow left cells without copies: nothing is mapped, and the build is repeated
-  const int n_real = (*A.err & (DERR_COPY_OVERFLOW | DERR_TILE_OVERFLOW | DERR_SCAN)) ? 0 : *A.n_real_dev;
+  const int n_real = (*A.err & kBuildFailed) ? 0 : *A.n_real_dev;
   const int SI = A.cell_split, SJ = A.stage_split;  // the host keeps cells x parts below 2^31
   const int S = SI * SJ;
   const int n_items = n_real * S;

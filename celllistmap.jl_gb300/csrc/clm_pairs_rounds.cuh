@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 4) ? 6 : 5)
   const int gw = blockIdx.x * kWarps + warp;
   const int nw = gridDim.x * kWarps;
   // a build that flagged an overflow left cells without copies: nothing is mapped, and the build is repeated
-  const int n_real = (*A.err & (DERR_COPY_OVERFLOW | DERR_TILE_OVERFLOW | DERR_SCAN)) ? 0 : *A.n_real_dev;
+  const int n_real = (*A.err & kBuildFailed) ? 0 : *A.n_real_dev;
   const int S = A.cell_split;  // the host keeps cells x parts below 2^31
   const int n_items = n_real * S;
   for (int r = gw; r < n_items; r += nw) {

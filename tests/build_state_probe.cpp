@@ -62,3 +62,37 @@ extern "C" void check_probe(int kind, int errw, int copies, int largest, int* ou
     out[4 + 3 * s] = S[s].small_cells == 0 && S[s].cell_count_zero == 0;
   }
 }
+
+// A sequence of steps of two sets built together: step k has the builds kind[k][s] (0 counting, 1 few particles, 2 bucket
+// of 24 places, 3 none) and the largest cells most[k][s]; each flags an overflow of its own set when the cell does not
+// fit.  state[k][s] after the step: small_off, bucket_off, bucket, dirty, tile_mult.
+extern "C" void crowding_probe(int n, const int* kind, const int* most, int* state) {
+  clm::BuildState S[2];
+  clm::BuildState* sets[2] = {&S[0], &S[1]};
+  for (int k = 0; k < n; k++) {
+    int words[64] = {};
+    for (int s = 0; s < 2; s++) {
+      const int kd = kind[2 * k + s], m = most[2 * k + s];
+      S[s].built = true;
+      S[s].dirty = false;
+      S[s].pending = kd != 3;
+      S[s].counted = true;
+      S[s].small = kd == 1;
+      S[s].bucket_used = kd == 2 ? std::max(24, S[s].bucket) : 0;
+      if (S[s].tile_mult == 0) S[s].tile_mult = 2;
+      S[s].cap_used = 1000;
+      words[32 + 2 * s] = 900;
+      words[44 + s] = kd == 1 && m <= clm::kBucket ? 0 : m;
+      if ((kd == 1 && m > clm::kBucket) || (kd == 2 && m > S[s].bucket_used)) words[40] |= clm::tile_overflow(s);
+    }
+    clm::check_builds(sets, 2, words);
+    for (int s = 0; s < 2; s++) {
+      int* o = state + 10 * k + 5 * s;
+      o[0] = S[s].small_off;
+      o[1] = S[s].bucket_off;
+      o[2] = S[s].bucket;
+      o[3] = S[s].dirty;
+      o[4] = S[s].tile_mult;
+    }
+  }
+}

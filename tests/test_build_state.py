@@ -48,3 +48,36 @@ def test_an_error_leaves_no_list_in_use(probe, kind, errw, status):
     for dirty, pending, cleared in (out[2:5], out[5:8]):
         assert dirty == (errw != 0)             # built again by the next call
         assert cleared == bool(errw & SCAN)     # and not on words that a block left half written
+
+
+def crowding(probe, kind, most):
+    n = len(kind)
+    out = (C.c_int * (10 * n))()
+    probe.crowding_probe(n, (C.c_int * (2 * n))(*sum(kind, [])), (C.c_int * (2 * n))(*sum(most, [])), out)
+    return [(tuple(out[10 * k:10 * k + 5]), tuple(out[10 * k + 5:10 * k + 10])) for k in range(n)]
+
+
+CLEAN = (0, 0, 0, 0, 2)
+
+
+@pytest.mark.parametrize("other", [0, 1, 2])
+@pytest.mark.parametrize("first", [0, 1])
+def test_an_overflow_is_one_sets_own(probe, other, first):
+    """The other set of the handle, whose cells fit, is not built again and keeps its builds."""
+    kind, most = [[1, other]], [[129, 20]]
+    if first:
+        kind, most = [[other, 1]], [[20, 129]]
+    st = crowding(probe, kind, most)[0]
+    assert st[first] == (1, 0, 168, 1, 2) and st[1 - first] == CLEAN
+
+
+def test_one_crowded_step_is_forgotten(probe):
+    """129 copies leave the small build for buckets of 168, 300 the buckets for the counting build; when the fullest
+    cell leaves a quarter free the builds are taken again, and not before."""
+    kind = [[1, 3], [2, 3], [2, 3], [2, 3], [0, 3], [0, 3], [0, 3], [2, 3], [1, 3]]
+    most = [[129, 0], [129, 0], [300, 0], [300, 0], [300, 0], [193, 0], [192, 0], [96, 0], [20, 0]]
+    got = [a for a, _ in crowding(probe, kind, most)]
+    assert [g[0] for g in got] == [1, 1, 1, 1, 1, 1, 1, 0, 0]       # small_off
+    assert [g[1] for g in got] == [0, 0, 1, 1, 1, 1, 0, 0, 0]       # bucket_off
+    assert got[0][2] == 168 and got[6][2] == 240 and got[7][2] == 120
+    assert all(g[4] == 2 for g in got)
