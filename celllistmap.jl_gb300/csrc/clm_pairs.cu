@@ -190,8 +190,9 @@ template <class T> struct FinishArgs {
   int nvec;                       // columns to sum: bins of a histogram, values of the adjoint
   const unsigned long long* part_hc;
   const double* part_hs;          // (the adjoint's values too)
-  unsigned long long* hc_out;     // histograms on the device: the caller's arrays
+  unsigned long long* hc_out;     // histograms on the device: the caller's arrays, written when no error is flagged
   double* hs_out;
+  const int* err;
   const unsigned long long* nl_count;
   unsigned char* res;             // pinned: layout of kResultBytes
   Totals totals;
@@ -227,9 +228,14 @@ template <class T, int N> __global__ void __launch_bounds__(kReduce) k_finish(co
       return;
     }
     const unsigned long long n = column_sum(F.part_hc, F.nb, F.nvec, c);
-    if (lead) {
-      (F.hc_out ? F.hc_out : reinterpret_cast<unsigned long long*>(F.res + 256))[c] = n;
-      (F.hs_out ? F.hs_out : reinterpret_cast<double*>(F.res + 256 + 8 * 256))[c] = s;
+    if (lead && F.hc_out) {
+      if (*F.err == 0) {  // the caller's arrays are left alone by a call that fails
+        F.hc_out[c] = n;
+        F.hs_out[c] = s;
+      }
+    } else if (lead) {
+      reinterpret_cast<unsigned long long*>(F.res + 256)[c] = n;
+      reinterpret_cast<double*>(F.res + 256 + 8 * 256)[c] = s;
     }
     return;
   }
@@ -395,6 +401,10 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
   if (hist) {
     if (!P || P->nbins < 1 || P->nbins > 256 || !P->bins || !P->vel_x || (h.nsets == 2 && !P->vel_y)) {
       h.last_error = "RHIST needs 1..256 bins, bin edges and velocities";
+      return ERR_ARG;
+    }
+    if (O->out_on_device && (!O->hist_count || !O->hist_sum)) {
+      h.last_error = "RHIST into device memory needs hist_count and hist_sum";
       return ERR_ARG;
     }
     need += align(sizeof(T) * (P->nbins + 1)) + align(sizeof(T) * nx * N) + align(sizeof(T) * ny * N);
@@ -597,6 +607,7 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
       if (O->out_on_device) {
         F.hc_out = reinterpret_cast<unsigned long long*>(O->hist_count);
         F.hs_out = O->hist_sum;
+        F.err = A.err;
       }
     }
     unsigned blocks = 1 + (unsigned)(F.nvec + kReduce / 32 - 1) / (kReduce / 32);
