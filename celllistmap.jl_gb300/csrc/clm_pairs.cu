@@ -261,7 +261,8 @@ static double estimated_pairs(const Handle& h, double vol) {
 
 // Parts per cell of the round-based kernel: cells holding many particles (large cutoff at high density) are
 // split into parts that take interleaved particle chunks, each at least two chunks of 32 particles, until there
-// are two items per resident warp slot (24 warps per SM).
+// are two items per resident warp slot (24 warps on each of a GB300's 152 SMs: fixed, as the order of the FP32 sums
+// depends on the parts).
 template <class T> int round_split_for(const Handle& h, const Geometry<T>& g) {
   const double nx = (double)h.sets[0].n;
   double real_cells = 1.0;
@@ -282,7 +283,7 @@ template <class T> int round_split_for(const Handle& h, const Geometry<T>& g) {
 // parts of its candidate stages, until there are `kItems` of them (a few per resident warp, so that the last ones
 // do not leave the others waiting) or a part is one chunk against one stage.  When even that leaves fewer
 // than 12 warps per SM with an item, the stages are made smaller.  Each part reads the cell's table and its
-// particles again, so not up to the full 24: a map of 32k Lennard-Jones particles takes 26.6 us with the line at 8
+// particles again, so not up to the full 24 (152: the SMs of a GB300; fixed, so that sums have one order): a map of 32k Lennard-Jones particles takes 26.6 us with the line at 8
 // or 12 warps and 30.7 us at 24, the closest pair of 1501 and 4507 points 26.4 us at 8 and 24.6 us at 12 or 24.
 struct ItemSplit {
   int si, sj, stage;

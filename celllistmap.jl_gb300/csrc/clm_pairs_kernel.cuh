@@ -109,9 +109,8 @@ __device__ __forceinline__ void pair_value(const PairArgs<T>& A, int op, V d2, i
 // Resident blocks per SM the kernel is compiled for.  Float64 lists and histograms take 128 registers (100k points: list
 // map 563 us, 620 at five blocks; histogram 47.1 ms, 48.1), Float64 forces do not gain by it (371 us, 379 at four).
 template <class T, int OPK, bool SPLIT> constexpr int min_blocks() {
-  if (sizeof(T) == 4) return OPK == OPK_ADJ ? 5 : 7;
-  if (SPLIT) return OPK == OPK_ADJ ? 4 : 5;
-  return (OPK == OPK_NL || OPK == OPK_HIST) ? 4 : 5;
+  if (sizeof(T) == 4) return 7;
+  return !SPLIT && (OPK == OPK_NL || OPK == OPK_HIST) ? 4 : 5;
 }
 
 // Shared memory of one warp.
@@ -161,6 +160,8 @@ template <class T, bool EXACT64, bool FP64, bool NL> struct WarpSmem {
 // OPC: the operator id when fixed at compile time, 0 = read from the arguments (9 only without types).
 template <class T, int N, int OPK, bool SPLIT, bool CROSS, bool BATCH, int OPC = 0>
 __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs(const __grid_constant__ PairArgs<T> A) {
+  static_assert(!in_rounds(OPK, std::is_same<T, double>::value, SPLIT, BATCH), "a map of k_pairs_rounds");
+  static_assert((OPK != OPK_HIST && OPK != OPK_ADJ) || (std::is_same<T, double>::value && !SPLIT), "FP64 sums");
   using V = T;
   using FA = typename std::conditional<std::is_same<T, double>::value && !SPLIT, double, float>::type;
   constexpr bool IS_F = (OPK == OPK_FORCES) || (OPK == OPK_ADJ);
@@ -770,32 +771,20 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
                   if (keep_pair(jp, ie, p4, q)) {
                     const int idx_i = idx_of(q.code_i), idx_j = idx_of(q.code_j);
                     // the bin from the FP32 distance, decided again from the IEEE distance of the reference's d2 when
-                    // an edge lies within 2^-12 of it (exact form: and the error of the FP32 distance of cell offsets)
+                    // an edge lies within 2^-12 and the error of the FP32 distance of cell offsets of it
                     bool exact_r = !q.sure;
-                    float rfl = 0.f;  // the distance in FP32 for the FP32 pair value
                     int b = -1;
                     if (q.sure) {
-                      rfl = sqrtf(q.d2f);
-                      const int lo = first_edge_at_or_above(s_binf, A.nbins, rfl);
+                      const float rf = sqrtf(q.d2f);
+                      const int lo = first_edge_at_or_above(s_binf, A.nbins, rf);
                       b = lo - 1;
-                      exact_r = near_edge(s_binf, A.nbins, lo, rfl, EXACT64 ? A.hist_err : 0.f);
+                      exact_r = near_edge(s_binf, A.nbins, lo, rf, A.hist_err);
                     }
-                    if (exact_r) {
-                      T e2;  // the reference's d2
-                      if constexpr (FP64) {
-                        if (!EXACT64 && q.sure) load_x(jp, ie, q);
-                        e2 = exact_d2<T, N>(q.dxs);
-                      } else {
-                        e2 = exact_d2<float, N>(q.dvf);
-                      }
-                      const T rr = xsqrt(e2);
-                      rfl = (float)rr;
-                      b = first_edge_at_or_above(s_bins, A.nbins, rr) - 1;
-                    }
+                    if (exact_r) b = first_edge_at_or_above(s_bins, A.nbins, xsqrt(exact_d2<T, N>(q.dxs))) - 1;
                     if (b >= 0 && b < A.nbins) {
                       FA dv[3] = {0, 0, 0};
 #pragma unroll
-                      for (int d = 0; d < N; d++) dv[d] = in_fp64(q) ? (FA)q.dxs[d] : (FA)q.dvf[d];
+                      for (int d = 0; d < N; d++) dv[d] = q.dxs[d];
                       if (tri) {
                         FA rv[3];
 #pragma unroll
@@ -809,20 +798,11 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
                         for (int a = 0; a < N; a++) dv[a] = rv[a];
                       }
                       FA dot = 0;
-                      if constexpr (std::is_same<FA, float>::value) {
-                        // FP32 pair values: velocities converted once by the host code
-                        const float* vy = CROSS ? A.vyf : A.vxf;
+                      const T* vy = CROSS ? A.vy : A.vx;
 #pragma unroll
-                        for (int d = 0; d < N; d++)
-                          dot += (A.vxf[(int64_t)idx_i * N + d] - vy[(int64_t)idx_j * N + d]) * dv[d];
-                        hv = dot * vrcp(rfl);
-                      } else {
-                        const T* vy = CROSS ? A.vy : A.vx;
-#pragma unroll
-                        for (int d = 0; d < N; d++)
-                          dot += ((FA)A.vx[(int64_t)idx_i * N + d] - (FA)vy[(int64_t)idx_j * N + d]) * dv[d];
-                        hv = dot * (FA)vrsqrt((double)value_d2(q));
-                      }
+                      for (int d = 0; d < N; d++)
+                        dot += (A.vx[(int64_t)idx_i * N + d] - vy[(int64_t)idx_j * N + d]) * dv[d];
+                      hv = dot * vrsqrt(value_d2(q));
                       hb = b;
                     }
                   }
@@ -1039,7 +1019,8 @@ cudaError_t launch_k(int& grid, cudaStream_t st, const PairArgs<T>& A) {
 
 // The potentials of the force and energy maps are known at compile time: the sweep's switch over the operators costs it
 // 4 to 12 % (100k points at cutoff 8, soft potential: forces 631 -> 602 us, energy 397 -> 369, split energy 141 -> 125,
-// split forces 274 -> 242).
+// split forces 274 -> 242).  Each is another set of kernels to compile, so the other operators, and Lennard-Jones forces
+// with type tables, take the switch.
 template <class T, int N, bool SPLIT, bool CROSS>
 cudaError_t launch_s(int opk, int& grid, cudaStream_t st, const PairArgs<T>& A) {
   switch (opk) {
