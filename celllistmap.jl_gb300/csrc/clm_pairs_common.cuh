@@ -33,8 +33,8 @@ template <class T> __device__ __forceinline__ T pos_of(const SetView<T>& S, int 
 //        Three and five FP64 instructions: GB300's FP64 pipe takes 16 cycles per warp instruction and bounds the
 //        FP64 pair kernels.  rsqrt.approx.f64 without .ftz is a sequence of its own: refined, it took 11 FP64
 //        slots and was within 1.7e-16 of 1/sqrt(x); this takes 5.7 and is within 1.2e-16 (3e9 values).  It takes
-//        subnormal x for zero, so those (distances below 1.5e-154) call the other form: the call costs the exact
-//        histograms 1 % (47.3 -> 47.9 ms), the same in line or as a predicated instruction 8 and 15 %.
+//        subnormal x for zero: pairs that close (1.5e-154) are evaluated apart (vrsqrt_tiny), as a test of x here costs
+//        the exact histograms 1 % as a call, 8 % in line and 15 % as a predicated instruction.
 __device__ __forceinline__ float vrcp(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -48,18 +48,18 @@ __device__ __forceinline__ double vrcp(double x) {
   e = fma(e, e, e);  // e + e^2
   return fma(y, e, y);
 }
-static __device__ __noinline__ double vrsqrt_subnormal(double x) {
-  double y;
-  asm("rsqrt.approx.f64 %0, %1;" : "=d"(y) : "d"(x));
-  return y;
-}
 __device__ __forceinline__ double vrsqrt(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  if (__double2hiint(x) < 0x00100000) y = vrsqrt_subnormal(x);
   const double e = fma(-x, y * y, 1.0);
   const double p = fma(0.375, e, 0.5);  // 1/2 + 3e/8
   return fma(y * e, p, y);
+}
+// For subnormal x, scaled by 2^108 (exactly).
+__device__ __forceinline__ double vrsqrt_tiny(double x) { return 0x1p54 * rsqrt(x * 0x1p108); }
+template <bool TINY, class V> __device__ __forceinline__ V vroot(V x) {
+  if constexpr (TINY) return (V)vrsqrt_tiny((double)x);
+  else return vrsqrt(x);
 }
 
 // a <= b and a < b for non-negative values (squared distances, the cutoff, +inf), decided on the bit

@@ -29,7 +29,8 @@ template <class V> struct LJTerm {
 
 // Per-pair energy u and g = (du/dr)/r (force contribution df = g*(x_i - x_j)).
 // OPC 9: LJ forces with one eps and sigma, whose products come from the host.
-template <class V, int OPC, class T>
+// TINY: d2 is subnormal.
+template <class V, int OPC, bool TINY = false, class T>
 __device__ __forceinline__ void pair_value(const PairArgs<T>& A, int op, V d2, int i, int j, V& u, V& g, LJTerm<V>& lj) {
   if constexpr (OPC == 9) {
     const V r2i = vrcp(d2);
@@ -49,16 +50,16 @@ __device__ __forceinline__ void pair_value(const PairArgs<T>& A, int op, V d2, i
       g = V(0);
       break;
     case 4:  // SUM_D
-      u = d2 * vrsqrt(d2);
+      u = d2 * vroot<TINY>(d2);
       g = V(0);
       break;
     case 5:  // SUM_INV_D
-      u = vrsqrt(d2);
+      u = vroot<TINY>(d2);
       g = V(0);
       break;
     case 6:
     case 7: {  // SOFT (c - d)^2
-      V ri = vrsqrt(d2);
+      V ri = vroot<TINY>(d2);
       V d = d2 * ri;
       V c = par<V>(A, 0);
       u = (c - d) * (c - d);
@@ -89,13 +90,13 @@ __device__ __forceinline__ void pair_value(const PairArgs<T>& A, int op, V d2, i
     }
     case 14: {  // weighted 1/d: u = -c w_i w_j / d, g = (c w_i w_j / d^2) / d
       const V cw = par<V>(A, 0) * weight<V>(A, false, i) * weight<V>(A, A.self == 0, j);
-      const V ri = vrsqrt(d2);
+      const V ri = vroot<TINY>(d2);
       u = -(cw * ri);
       g = cw * (ri * ri * ri);
       break;
     }
     case 12: {  // 1/d with gradient accumulation
-      V ri = vrsqrt(d2);
+      V ri = vroot<TINY>(d2);
       u = ri;
       g = ri * ri * ri;
       break;
@@ -168,6 +169,8 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
   constexpr bool FP64 = std::is_same<T, double>::value;
   constexpr bool EXACT64 = FP64 && !SPLIT;  // pair values in FP64 from the coordinates themselves
   constexpr bool ABS_PF = !FP64;            // Float32 handles test the coordinates themselves
+  // the operator may take the root of an FP64 d2: pairs too close for it (thr_tiny) are decided one by one
+  constexpr bool ROOT = EXACT64 && ((OPK == OPK_SCALAR && OPC != 8) || (OPK == OPK_FORCES && OPC != 9) || OPK == OPK_HIST);
   const DevGeom<T>& g = A.g;
   const int op = OPC ? OPC : A.op;
   using Smem = WarpSmem<T, EXACT64, FP64, OPK == OPK_NL>;
@@ -468,6 +471,54 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
               }
             }
           };
+          // d2 of a kept pair in FP64 for values (fused; the decision is made): EXACT64, or Float64 handles near the
+          // cutoff
+          auto value_d2 = [&](const Pair& q) {
+            T d2 = q.dxs[0] * q.dxs[0];
+#pragma unroll
+            for (int d = 1; d < N; d++) d2 = fma(q.dxs[d], q.dxs[d], d2);
+            return d2;
+          };
+          // A kept pair whose d2 is subnormal, evaluated by itself.
+          auto is_tiny = [](T d2) { return d2 > T(0) && d2 < T(0x1p-1022); };
+          auto tiny_pair = [&](const Pair& q) {
+            const int idx_i = idx_of(q.code_i), idx_j = idx_of(q.code_j);
+            const bool sw = sym && idx_j < idx_i;
+            if constexpr (OPK == OPK_HIST) {
+              const int b = first_edge_at_or_above(s_bins, A.nbins, xsqrt(exact_d2<T, N>(q.dxs))) - 1;
+              if (b < 0 || b >= A.nbins) return;
+              const T* vy = CROSS ? A.vy : A.vx;
+              FA dot = 0;
+#pragma unroll
+              for (int a = 0; a < N; a++) {
+                FA x = q.dxs[a];
+                if (tri) {
+                  x = 0;
+#pragma unroll
+                  for (int k = 0; k < N; k++) x += (FA)gc.Rinv[a][k] * q.dxs[k];
+                }
+                dot += (A.vx[(int64_t)idx_i * N + a] - vy[(int64_t)idx_j * N + a]) * x;
+              }
+              atomicAdd(&s_hc[b], 1ull);
+              atomicAdd(&s_hs[b], (double)(dot * vroot<true>(value_d2(q))));
+            } else {
+              V u, gg;
+              LJTerm<V> lv;
+              pair_value<V, OPC, true>(A, op, value_d2(q), sw ? idx_j : idx_i, sw ? idx_i : idx_j, u, gg, lv);
+              if (op == 2) c_acc++;
+              else e_part += (FA)u;
+              if constexpr (OPK == OPK_FORCES) {
+                FA df[3] = {0, 0, 0}, nf[3] = {0, 0, 0};
+#pragma unroll
+                for (int d = 0; d < N; d++) {
+                  df[d] = (FA)(gg * q.dxs[d]);
+                  nf[d] = -df[d];
+                }
+                force_add<T, N, FA>(A, false, idx_i, nf);
+                force_add<T, N, FA>(A, CROSS, idx_j, df);
+              }
+            }
+          };
           // Whether the reference keeps the pair.  The rest of the pair rules on the codes (image: negative code
           // ~index): pairs of two images are dropped; in triclinic self pairs of a real copy and an image, the copy of
           // the lower index is the reference's i and must be real, so with r the real copy's index and m the
@@ -481,7 +532,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
             q.d2f = fmaf(q.dvf[2], q.dvf[2], fmaf(q.dvf[1], q.dvf[1], q.dvf[0] * q.dvf[0]));
             if constexpr (EXACT64) load_x(jp, ie, q);
             const int drop = (q.code_i & q.code_j) | ((q.code_i ^ q.code_j) & ~(q.code_i + q.code_j + 1) & sym_mask);
-            q.sure = q.d2f <= g.thr_lo;
+            q.sure = q.d2f <= g.thr_lo && (!ROOT || q.d2f >= g.thr_tiny);
             if (drop < 0 || !q.sure) {
               if (drop < 0) return false;
               const int e = w0 + jp - ((jp / kPad) << 2);
@@ -490,8 +541,15 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
               const int3 c3 = make_int3(ci[0], ci[1], ci[2]);
               if constexpr (FP64) {
                 if constexpr (!EXACT64) load_x(jp, ie, q);
-                return near_cutoff<T, N>(gc, g.cutoff_sqr, c3, W.meta[lo], e < same_end, sw, q.xi[0], q.xi[1],
-                                         (N == 3) ? q.xi[2] : T(0), q.xj[0], q.xj[1], (N == 3) ? q.xj[2] : T(0));
+                const bool in = near_cutoff<T, N>(gc, g.cutoff_sqr, c3, W.meta[lo], e < same_end, sw, q.xi[0], q.xi[1],
+                                                  (N == 3) ? q.xi[2] : T(0), q.xj[0], q.xj[1], (N == 3) ? q.xj[2] : T(0));
+                if constexpr (ROOT) {
+                  if (in && is_tiny(value_d2(q))) {
+                    tiny_pair(q);
+                    return false;
+                  }
+                }
+                return in;
               } else {
                 q.d2f = exact_d2<float, N>(q.dvf);
                 return near_cutoff<T, N>(gc, g.cutoff_sqr, c3, W.meta[lo], e < same_end, sw, p4.x, p4.y, p4.z,
@@ -499,14 +557,6 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
               }
             }
             return true;
-          };
-          // d2 of a kept pair in FP64 for values (fused; the decision is made): EXACT64, or Float64 handles near the
-          // cutoff
-          auto value_d2 = [&](const Pair& q) {
-            T d2 = q.dxs[0] * q.dxs[0];
-#pragma unroll
-            for (int d = 1; d < N; d++) d2 = fma(q.dxs[d], q.dxs[d], d2);
-            return d2;
           };
           // values in FP64: always (EXACT64), never (Float32 handles), or near the cutoff (split form)
           auto in_fp64 = [&](const Pair& q) { return EXACT64 || (FP64 && !q.sure); };
@@ -676,7 +726,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
                   if (in_fp64(q)) {
                     V uv, gv;
                     LJTerm<V> lv;
-                    pair_value<V, OPC, T>(A, op, value_d2(q), oi, oj, uv, gv, lv);
+                    pair_value<V, OPC>(A, op, value_d2(q), oi, oj, uv, gv, lv);
                     uu = (FA)uv;
                     gg = (FA)gv;
                     lj.from(lv);
@@ -685,7 +735,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
                   } else {
                     float uf, gf;
                     LJTerm<float> lv;
-                    pair_value<float, OPC, T>(A, op, q.d2f, oi, oj, uf, gf, lv);
+                    pair_value<float, OPC>(A, op, q.d2f, oi, oj, uf, gf, lv);
                     uu = (FA)uf;
                     gg = (FA)gf;
                     lj.from(lv);
@@ -731,12 +781,12 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
                   } else if (in_fp64(q)) {
                     V uu, gg;
                     LJTerm<V> lv;
-                    pair_value<V, OPC, T>(A, op, value_d2(q), oi, oj, uu, gg, lv);
+                    pair_value<V, OPC>(A, op, value_d2(q), oi, oj, uu, gg, lv);
                     e_part += (FA)uu;
                   } else {
                     float uu, gg;
                     LJTerm<float> lv;
-                    pair_value<float, OPC, T>(A, op, q.d2f, oi, oj, uu, gg, lv);
+                    pair_value<float, OPC>(A, op, q.d2f, oi, oj, uu, gg, lv);
                     e_part += (FA)uu;
                   }
                 }

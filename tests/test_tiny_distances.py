@@ -15,3 +15,29 @@ def test_values_at_tiny_distances(clm, d):
         got = clm.pairwise(op, s)
         assert abs(got - want) <= 1e-12 * want, (op.op, got, want)
     s.close()
+
+
+@pytest.mark.parametrize("cross", [False, True])
+@pytest.mark.parametrize("d", [0.8e-154, 1.4e-154, 1.0e-150])
+def test_forces_and_histogram_at_tiny_distances(clm, d, cross):
+    x = np.array([[0.0, 0.0, 0.0], [d, 0.0, 0.0], [9.0, 9.0, 9.0]])
+    p = {"xpositions": x}
+    if cross:
+        p = {"xpositions": x[[0, 2]], "ypositions": x[[1]]}
+    s = clm.ParticleSystem(**p, unitcell=None, cutoff=1.0)
+    u = (d / np.sqrt(d * d))  # 1 but for the bits that a subnormal d2 lacks
+    ef = clm.pairwise(clm.SoftForces(), s)
+    assert abs(ef.energy - 1.0) <= 1e-12
+    want = np.zeros_like(p["xpositions"])
+    want[0, 0] = -2.0 * u
+    if cross:
+        np.testing.assert_allclose(ef.forces_y, [[2.0 * u, 0.0, 0.0]], rtol=1e-12)
+    else:
+        want[1, 0] = 2.0 * u
+    np.testing.assert_allclose(ef.forces, want, rtol=1e-12)
+    v = np.array([[3.0, 1.0, 2.0], [1.0, 5.0, 2.0], [0.0, 0.0, 0.0]])
+    vel = (v[[0, 2]], v[[1]]) if cross else (v,)
+    hc, hs = clm.pairwise(clm.RadialHistogram(np.array([0.0, 0.5, 1.0]), *vel), s)
+    assert hc.tolist() == [1, 0]
+    np.testing.assert_allclose(hs, [-2.0 * u, 0.0], rtol=1e-12)
+    s.close()
