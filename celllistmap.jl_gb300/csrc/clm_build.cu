@@ -825,11 +825,12 @@ __global__ void __launch_bounds__(kBlock) k_bucket_gather(const __grid_constant_
 // value (particle-index order) and gather them.  A cell with more than kBucket copies is flagged
 // (tile_overflow) and the set is built by the other kernels until its cells are emptier again (check_builds).
 // Not one cooperative launch with a barrier over its grid: that waits until the device has room for all of its blocks at
-// once, and never starts beside a kernel that holds most of the multiprocessors until this step is done.  It built 1 to
-// 2 us faster (32,000 particles 22 / 27 us); the steps of 1,003 and 32,000 particles took the same time (82 and 76 us).
+// once, and never starts beside a kernel that holds most of the multiprocessors until this step is done.  The second
+// kernel is set up while the first runs: 32,000 Float32 / Float64 particles take 20.7 / 24.9 us, 22.6 / 27.5 us one after
+// the other, and took 21.9 / 26.6 us in the cooperative launch.
 constexpr int kSmallThreads = 512;
-// Up to here this is the shorter build (GB300, Float32 / Float64 at liquid density: 4,000 particles 19 / 22 us against
-// 28 / 33 of the bucket build, 32,000 23 / 28 against 30 / 35, 65,536 28 / 36 against 32 / 39 for one particle more).
+// Up to here this is the shorter build (GB300, Float32 / Float64 at liquid density: 4,000 particles 16 / 19 us against
+// 28 / 33 of the bucket build, 32,000 21 / 25 against 30 / 35, 65,536 26 / 33 against 32 / 39 for one particle more).
 constexpr int64_t kSmallParticles = 1 << 16;
 constexpr int64_t kSmallCells = 1 << 15;
 constexpr double kSmallPerCell = 64.0;  // copies per cell expected at uniform density: half a bucket
@@ -870,6 +871,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_place(const __grid_cons
   int block, blocks;
   const SmallSet<T>& B = small_set(A, block, blocks);
   __shared__ PlaceShared<T, N, kSmallThreads> sm;
+  cudaTriggerProgrammaticLaunchCompletion();  // k_small_cells may be set up; it waits for the end of this kernel
   load_shift<T>(A.g, sm.shift);
   if (block == 0 && threadIdx.x == 0) *B.max_cell = 0;
   for (int c = block * kSmallThreads + threadIdx.x; c < 2 * B.ncells; c += blocks * kSmallThreads) B.cf_next[c] = 0;
@@ -888,6 +890,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_cells(const __grid_cons
   constexpr int kW = kSmallThreads / 32;
   __shared__ T s_shift[27][3];
   load_shift<T>(g, s_shift);
+  cudaGridDependencySynchronize();
   const int per = (B.ncells + blocks - 1) / blocks;
   const int c0 = min(B.ncells, block * per), c1 = min(B.ncells, c0 + per);
   __shared__ int s_sum[2][kW];
@@ -1346,8 +1349,17 @@ template <class T> int launch_small(Handle& h, SmallBuild<T>& A, unsigned which,
   place<<<(unsigned)blocks, kSmallThreads, 0, h.stream>>>(A);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) {
-    cells<<<(unsigned)blocks, kSmallThreads, 0, h.stream>>>(A);
-    e = cudaGetLastError();
+    // set up while k_small_place runs (every block of that one has begun by then, so it cannot be kept from ending)
+    cudaLaunchAttribute overlap = {};
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.stream = h.stream;
+    cfg.attrs = &overlap;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, cells, A);
   }
   for (int s = 0; s < h.nsets; s++)
     if (which >> s & 1u) small_launched(h.sets[s], h.sets[s].ncells, e == cudaSuccess);
