@@ -482,6 +482,7 @@ template <class T> int run_pairs(Handle& h, const Geometry<T>& g, int op, const 
     } else {
       for (size_t k = 0; k < b.size(); k++) b[k] = (T)P->bins[k];
     }
+    A.first_edge = (double)b[0];
     CLM_CUDA_TRY(h, cudaMemcpyAsync(bins, b.data(), sizeof(T) * b.size(), cudaMemcpyHostToDevice, h.stream));
     CLM_CUDA_TRY(h, cudaMemcpyAsync(vx, P->vel_x, sizeof(T) * nx * N, k_in, h.stream));
     if (ny) CLM_CUDA_TRY(h, cudaMemcpyAsync(vy, P->vel_y, sizeof(T) * ny * N, k_in, h.stream));

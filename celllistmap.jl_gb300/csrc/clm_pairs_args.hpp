@@ -62,6 +62,7 @@ template <class T> struct PairArgs {
   const T* vy;
   const T* bins;
   int nbins;
+  double first_edge;  // bins[0], on the host
   const float* vxf;  // velocities in FP32 (pair values of the FP32 forms)
   const float* vyf;
   const double* wx;   // per-particle weights (WEIGHTED_INV_D) of x and y, and FP32 copies

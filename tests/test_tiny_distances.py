@@ -37,7 +37,11 @@ def test_forces_and_histogram_at_tiny_distances(clm, d, cross):
     np.testing.assert_allclose(ef.forces, want, rtol=1e-12)
     v = np.array([[3.0, 1.0, 2.0], [1.0, 5.0, 2.0], [0.0, 0.0, 0.0]])
     vel = (v[[0, 2]], v[[1]]) if cross else (v,)
-    hc, hs = clm.pairwise(clm.RadialHistogram(np.array([0.0, 0.5, 1.0]), *vel), s)
-    assert hc.tolist() == [1, 0]
-    np.testing.assert_allclose(hs, [-2.0 * u, 0.0], rtol=1e-12)
+    for first in (0.0, -0.3, -1.0e-9):
+        hc, hs = clm.pairwise(clm.RadialHistogram(np.array([first, 0.5, 1.0]), *vel), s)
+        assert hc.tolist() == [1, 0]
+        np.testing.assert_allclose(hs, [-2.0 * u, 0.0], rtol=1e-12)
+    for first in (0.01, 3.0e-154, 2.9e-154):  # either side of the line above which tiny distances are not looked for
+        want = [int(d > first), 0]
+        assert clm.pairwise(clm.RadialHistogram(np.array([first, 0.5, 1.0]), *vel), s)[0].tolist() == want
     s.close()
