@@ -167,9 +167,6 @@ template <class T> void fill_devgeom(const Geometry<T>& g, int precision, DevGeo
   double c2 = (double)g.cutoff_sqr;
   d.thr_hi = std::nextafter((float)(c2 * (1.0 + std::ldexp(1.0, -13))), INFINITY);
   d.thr_lo = std::nextafter((float)(c2 * (1.0 - std::ldexp(1.0, -13))), 0.0f);
-  // Coordinates whose exact d2 is subnormal (below 2^-1022) are within 2^-960 of each other and of zero in every dimension
-  // that they differ in: their FP32 distance is rounding only, some 2^-20 of a cell side.  The line is far above that.
-  d.thr_tiny = (float)(c2 * std::ldexp(1.0, -30));
   // The projection filter compares |proj_i - proj_j| <= d with the cutoff, and |proj_j| <= (a particle's share of its
   // cell) + d with the margin: in exact arithmetic it keeps every pair of d <= cutoff, and it rejects one only by the
   // rounding of coordinates, cell centres and dot products, about 20 units of the largest coordinate and the cutoff.

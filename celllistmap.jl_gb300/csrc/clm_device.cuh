@@ -151,7 +151,6 @@ template <class T> struct DevGeom {
   float csf_lo[3];      // cell size - csf (low part of the float pair)
   float cbf_hi[3], cbf_lo[3];  // computing-box minimum as a float pair
   float thr_hi, thr_lo; // FP32 prefilter bounds on d2 (maybe-inside / surely-inside)
-  float thr_tiny;       // FP32 d2 from which on the Float64 d2 is a normal number
   T proj_lo;            // the projection filter keeps every pair of d2 up to this (>= thr_lo)
   int zero_code;        // image code of the zero shift (13 in 3D, 4 in 2D)
   int nimg;             // 3^dim

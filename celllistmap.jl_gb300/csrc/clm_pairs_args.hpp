@@ -62,7 +62,6 @@ template <class T> struct PairArgs {
   const T* vy;
   const T* bins;
   int nbins;
-  double first_edge;  // bins[0], on the host
   const float* vxf;  // velocities in FP32 (pair values of the FP32 forms)
   const float* vyf;
   const double* wx;   // per-particle weights (WEIGHTED_INV_D) of x and y, and FP32 copies
@@ -97,9 +96,13 @@ template <class T> struct PairArgs {
   const DevGeom<T>* gtab;       // batch: geometry of each system
   const int* cell_sys;          // batch: system of each global cell
   const int* cbase;             // batch: first global cell of each system
+  double first_edge;            // RHIST: bins[0], for the host
+  float thr_tiny;               // FP32 d2 from which on the Float64 d2 is a normal number (set_params)
 };
 
-// Operator parameters in both precisions.
+// Operator parameters in both precisions, and the line below which a pair's root may not be taken from its estimate:
+// coordinates whose exact d2 is subnormal (below 2^-1022) are within 2^-960 of each other and of zero in every dimension
+// that they differ in, so their FP32 distance is rounding only, some 2^-20 of a cell side; the line is far above that.
 template <class T> inline void set_params(PairArgs<T>& A, const double* p) {
   for (int k = 0; k < 4; k++) {
     A.p[k] = p[k];
@@ -112,6 +115,7 @@ template <class T> inline void set_params(PairArgs<T>& A, const double* p) {
     o[3] = 12 * o[1];
     o[4] = 6 * o[2];
   };
+  A.thr_tiny = (float)((double)A.g.cutoff_sqr * 0x1p-30);
   lj(A.ljd, A.p);
   lj(A.ljf, A.pf);
 }

@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks<T, OPK, SPLIT>()) k_pairs
             q.d2f = fmaf(q.dvf[2], q.dvf[2], fmaf(q.dvf[1], q.dvf[1], q.dvf[0] * q.dvf[0]));
             if constexpr (EXACT64) load_x(jp, ie, q);
             const int drop = (q.code_i & q.code_j) | ((q.code_i ^ q.code_j) & ~(q.code_i + q.code_j + 1) & sym_mask);
-            q.sure = q.d2f <= g.thr_lo && (!ROOT || q.d2f >= g.thr_tiny);
+            q.sure = q.d2f <= g.thr_lo && (!ROOT || q.d2f >= A.thr_tiny);
             if (drop < 0 || !q.sure) {
               if (drop < 0) return false;
               const int e = w0 + jp - ((jp / kPad) << 2);
